@@ -272,9 +272,11 @@ void ef_destroy(ef_ctx* c) {
     F(c->dKvijTmp);
     F(c->dPart);
     F(c->dRed);
-    F(c->dPartA);
-    F(c->dPartB);
-    F(c->dBar);
+    F(c->dPcgSlots);
+    F(c->dPcgHaloPtr);
+    F(c->dPcgHaloIdx);
+    F(c->dPcgGroupPtr);
+    F(c->dPcgLcol);
     F(c->dPcgRes);
     for (auto* p : c->w32) F(p);
     for (auto* p : c->w64) F(p);
@@ -913,15 +915,9 @@ ef_status ef_finalize(ef_ctx* c, int options) {
     c->dPart = dalloc<double>(4 * c->nPart, &st);
     c->dRed = dalloc<double>(16, &st);
     if (!c->dPart || !c->dRed) return st;
-    EF_CHECK(ef_pcg_grid(0, c->nSM, &c->pcgGrid[0]));
-    EF_CHECK(ef_pcg_grid(1, c->nSM, &c->pcgGrid[1]));
-    const int maxGrid = std::max(c->pcgGrid[0], c->pcgGrid[1]);
-    c->dPartA = dalloc<double>(4 * (size_t)maxGrid, &st);
-    c->dPartB = dalloc<double>(4 * (size_t)maxGrid, &st);
-    c->dBar = dalloc<char>(ef_barrier_state_bytes(), &st);
+    c->dPcgSlots = dalloc<double>(ef_pcg_slot_bytes(ef_pcg_slot_sets()) / sizeof(double), &st);
     c->dPcgRes = dalloc<char>(ef_pcg_result_bytes(), &st);
-    if (!c->dPartA || !c->dPartB || !c->dBar || !c->dPcgRes) return st;
-    EF_CUDA(cudaMemset(c->dBar, 0, ef_barrier_state_bytes()));
+    if (!c->dPcgSlots || !c->dPcgRes) return st;
     for (int i = 0; i < 7; ++i) {
         c->w32[i] = dalloc<float>(c->nDof, &st);
         if (!c->w32[i]) return st;

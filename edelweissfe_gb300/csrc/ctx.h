@@ -16,19 +16,25 @@
 #include <vector>
 
 #include "ef_common.cuh"
+#include "pcg_plan.h"
 
 // krylov.cu
 int ef_krylov_block_threads();
-size_t ef_barrier_state_bytes();
+int ef_pcg_slot_sets();
+size_t ef_pcg_slot_bytes(int sets);
 size_t ef_pcg_result_bytes();
 ef_status ef_launch_bsr_residual(int nNodes, const int32_t* rowPtr, const int32_t* colIdx, const void* vals,
                                  int mDouble, const double* x, const double* b, const uint8_t* mask, double* y,
                                  int nSM, cudaStream_t s);
-ef_status ef_pcg_grid(int vDouble, int nSM, int* gridOut);
-ef_status ef_launch_pcg(int vDouble, int grid, int nNodes, const int32_t* rowPtr, const int32_t* colIdx,
+ef_status ef_launch_pcg(int vDouble, int nSM, int nNodes, const int32_t* rowPtr, const int32_t* colIdx,
                         const void* vals, const void* binv, const uint8_t* mask, const void* b, void* x, void* r,
-                        void* z, void* pA, void* pB, void* q, double* partA, double* partB, void* bar, void* res,
-                        int maxIter, double rtol2, int* flags, cudaStream_t s);
+                        void* z, void* pA, void* pB, void* q, double* slots, int slotSets, void* res, int maxIter,
+                        double rtol2, int* flags, cudaStream_t s);
+ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes, const int32_t* rowPtr,
+                                 const uint16_t* lcol, const int32_t* haloPtr, const int32_t* haloIdx,
+                                 const int32_t* groupPtr, size_t smem, const void* vals, const void* binv,
+                                 const uint8_t* mask, const void* b, void* x, void* z, double* slots, void* res,
+                                 int maxIter, double rtol2, int* flags, cudaStream_t s);
 ef_status ef_launch_dot(int64_t n, const double* a, const double* b, double* part, int nPart, double* out,
                         cudaStream_t s);
 ef_status ef_launch_masked_copy(int64_t n, const double* src, const uint8_t* mask, int keepMasked, double scale,
@@ -415,9 +421,14 @@ struct ef_ctx {
     double* dPart = nullptr;
     int nPart = 0;
     double* dRed = nullptr;  // small result buffer
-    int pcgGrid[2] = {0, 0};
-    double *dPartA = nullptr, *dPartB = nullptr;
-    void* dBar = nullptr;
+    double* dPcgSlots = nullptr;  // reduction slots of the persistent PCG
+    // resident PCG (ef_pcg_resident_plan), made at the context's first PCG solve; the system has one
+    // precision, so one plan: 0 bytes of shared memory: the streaming kernel
+    bool pcgPlanned = false;
+    size_t pcgSmem = 0;
+    PcgShape pcgShape;
+    int32_t *dPcgHaloPtr = nullptr, *dPcgHaloIdx = nullptr, *dPcgGroupPtr = nullptr;
+    uint16_t* dPcgLcol = nullptr;
     void* dPcgRes = nullptr;
     void* w32[7] = {};  // FP32 Krylov vectors: b, x, r, z, p (two buffers), q
     double* w64[5] = {};  // FP64: xd, xf, r64, tmp, y

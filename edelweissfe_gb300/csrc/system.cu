@@ -155,15 +155,37 @@ ef_status dot_host(ef_ctx* c, const double* a, const double* b, double* out, cud
     return EF_OK;
 }
 
-// one PCG launch on the free DOFs: solves K d = rhs (rhs zero on Dirichlet DOFs)
+static ef_status pcg_plan(ef_ctx* c, int vDouble) {
+    if (c->pcgPlanned) return EF_OK;
+    PcgResidentPlan p;
+    ef_pcg_resident_plan(vDouble, c->nSM, (int)c->nNodes, c->hRowPtr0.data(), c->hColIdx0.data(), p);
+    if (p.smem > 0) {
+        EF_CHECK(upload(&c->dPcgHaloPtr, p.haloPtr));
+        EF_CHECK(upload(&c->dPcgHaloIdx, p.haloIdx));
+        EF_CHECK(upload(&c->dPcgGroupPtr, p.groupPtr));
+        EF_CHECK(upload(&c->dPcgLcol, p.lcol));
+    }
+    c->pcgSmem = p.smem;
+    c->pcgShape = p.shape;
+    c->pcgPlanned = true;
+    return EF_OK;
+}
+
+// one PCG launch on the free DOFs: solves K d = rhs (rhs zero on Dirichlet DOFs); vDouble: the
+// precision of the system
 ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol,
                          PcgResultHost* out, ef_solve_info* prof, cudaStream_t s) {
     void** w = vDouble ? c->w64k : c->w32;
-    EF_CUDA(cudaMemsetAsync(c->dBar, 0, ef_barrier_state_bytes(), s));
+    EF_CHECK(pcg_plan(c, vDouble));
     if (prof) EF_CUDA(cudaEventRecord(c->ev[0], s));
-    EF_CHECK(ef_launch_pcg(vDouble, c->pcgGrid[vDouble], (int)c->nNodes, c->dRowPtr, c->dColIdx, c->dBsrVals, c->dBinv,
-                           c->dMask, rhs, sol, w[2], w[3], w[4], w[5], w[6], c->dPartA, c->dPartB, c->dBar,
-                           c->dPcgRes, maxIter, rtol * rtol, c->dFlags, s));
+    if (c->pcgSmem > 0)
+        EF_CHECK(ef_launch_pcg_resident(vDouble, c->pcgShape, (int)c->nNodes, c->dRowPtr, c->dPcgLcol, c->dPcgHaloPtr,
+                                        c->dPcgHaloIdx, c->dPcgGroupPtr, c->pcgSmem, c->dBsrVals, c->dBinv, c->dMask,
+                                        rhs, sol, w[3], c->dPcgSlots, c->dPcgRes, maxIter, rtol * rtol, c->dFlags, s));
+    else
+        EF_CHECK(ef_launch_pcg(vDouble, c->nSM, (int)c->nNodes, c->dRowPtr, c->dColIdx, c->dBsrVals, c->dBinv, c->dMask,
+                               rhs, sol, w[2], w[3], w[4], w[5], w[6], c->dPcgSlots, ef_pcg_slot_sets(), c->dPcgRes,
+                               maxIter, rtol * rtol, c->dFlags, s));
     if (prof) EF_CUDA(cudaEventRecord(c->ev[1], s));
     EF_CUDA(cudaMemcpyAsync(out, c->dPcgRes, sizeof(PcgResultHost), cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));
