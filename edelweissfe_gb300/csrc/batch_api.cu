@@ -3,6 +3,76 @@
 
 #include "ctx.h"
 
+static const int kBatchLanes[3] = {1, 4, 8};
+
+// the sliced layouts of the batched PCG for 1, 4 and 8 lanes per block row; their values and columns share one
+// buffer, which every solve fills for its tile's lanes
+static ef_status batch_plans(ef_ctx* c, int nProb, const int32_t* nodePtr) {
+    for (void* p : c->batchMem) cudaFree(p);
+    c->batchMem.clear();
+    int64_t most = 1;
+    auto keep = [&](const std::vector<int32_t>& v, const int32_t** out) -> ef_status {
+        int32_t* d = nullptr;
+        EF_CHECK(upload(&d, v));
+        c->batchMem.push_back(d);
+        *out = d;
+        return EF_OK;
+    };
+    for (int i = 0; i < 3; ++i) {
+        const int lpr = kBatchLanes[i], rpw = 32 / lpr;
+        std::vector<int32_t> base(nProb), ptr, row, end, step;
+        int64_t steps = 0;
+        for (int p = 0; p < nProb; ++p) {
+            base[p] = (int32_t)ptr.size();
+            for (int32_t m0 = nodePtr[p]; m0 < nodePtr[p + 1]; m0 += rpw) {
+                int w = 0;
+                for (int32_t m = m0; m < std::min(nodePtr[p + 1], m0 + rpw); ++m)
+                    w = std::max(w, (c->hRowPtr0[m + 1] - c->hRowPtr0[m] + lpr - 1) / lpr);
+                ptr.push_back((int32_t)steps);
+                row.push_back(m0);
+                end.push_back(nodePtr[p + 1]);
+                step.push_back((int32_t)steps);
+                steps += w;
+                step.push_back((int32_t)steps);
+            }
+            ptr.push_back((int32_t)steps);
+        }
+        if (steps >= ((int64_t)1 << 31)) {
+            ef_set_error("ef_batch_setup: too many blocks");
+            return EF_ERR_ARG;
+        }
+        BatchPlanDev& pl = c->batchPlan[i];
+        pl = BatchPlanDev();
+        pl.nGroups = (int)row.size();
+        pl.nodePtr = c->dBatchNodePtr;
+        pl.order = c->dBatchOrder;
+        EF_CHECK(keep(base, &pl.groupBase));
+        EF_CHECK(keep(ptr, &pl.groupPtr));
+        EF_CHECK(keep(row, &pl.groupRow));
+        EF_CHECK(keep(end, &pl.groupEnd));
+        EF_CHECK(keep(step, &pl.groupStep));
+        most = std::max(most, steps);
+    }
+    ef_status st = EF_OK;
+    double* vals = dalloc<double>((size_t)288 * most, &st);
+    if (!vals) return st;
+    c->batchMem.push_back(vals);
+    int32_t* col = dalloc<int32_t>((size_t)32 * most, &st);
+    if (!col) return st;
+    c->batchMem.push_back(col);
+    c->dBatchTicket = dalloc<int>(1, &st);
+    if (!c->dBatchTicket) return st;
+    c->batchMem.push_back(c->dBatchTicket);
+    for (BatchPlanDev& pl : c->batchPlan) {
+        pl.vals = vals;
+        pl.col = col;
+    }
+    std::vector<int> sizes(nProb);
+    for (int p = 0; p < nProb; ++p) sizes[p] = nodePtr[p + 1] - nodePtr[p];
+    c->batchCluster = ef_batch_cluster_size(c->nSM, sizes);
+    return EF_OK;
+}
+
 ef_status ef_batch_setup(ef_ctx* c, int nProb, const int32_t* nodePtr) {
     EF_REQUIRE_FINALIZED(c);
     if (nProb <= 0 || !nodePtr || nodePtr[0] != 0 || nodePtr[nProb] != (int32_t)c->nNodes) {
@@ -41,6 +111,8 @@ ef_status ef_batch_setup(ef_ctx* c, int nProb, const int32_t* nodePtr) {
     if (st != EF_OK) return st;
     EF_CUDA(cudaMemcpy(c->dBatchNodePtr, nodePtr, sizeof(int32_t) * (nProb + 1), cudaMemcpyHostToDevice));
     EF_CUDA(cudaMemcpy(c->dBatchOrder, order.data(), sizeof(int32_t) * nProb, cudaMemcpyHostToDevice));
+    c->batchN = 0;
+    EF_CHECK(batch_plans(c, nProb, nodePtr));
     c->batchN = nProb;
     return EF_OK;
 }
@@ -71,11 +143,14 @@ static ef_status batch_solve(ef_ctx* c, int tile, double rtol, int maxIter, cons
     // Dirichlet DOFs take b; the free part solves K_ff x_f = b_f - K_fd x_d per problem
     EF_CHECK(ef_launch_masked_copy(n, b, c->dMask, 1, 1.0, xd, 1, s));
     EF_CHECK(residual64(c, xd, b, r64, s));
-    double* w[5];
-    for (int i = 0; i < 5; ++i) w[i] = (double*)c->w64k[1 + i];
-    EF_CHECK(ef_launch_batched_pcg(tile, c->nSM, c->batchN, c->dBatchNodePtr, c->dBatchOrder, c->dRowPtr, c->dColIdx,
-                                   (const double*)c->dBsrVals, (const double*)c->dBinv, c->dMask, r64, w[0], w[1],
-                                   w[2], w[3], w[4], maxIter, rtol * rtol, iters, relres, s));
+    double* w[6];
+    for (int i = 0; i < 6; ++i) w[i] = (double*)c->w64k[1 + i];
+    int tpb = 0, lpr = 0;
+    ef_batch_tile_shape(tile, &tpb, &lpr);
+    EF_CHECK(ef_launch_batched_pcg(tile, c->batchPlan[lpr == 1 ? 0 : (lpr == 4 ? 1 : 2)], c->batchCluster, c->nSM, c->batchN,
+                                   c->dRowPtr, c->dColIdx, (const double*)c->dBsrVals, (const double*)c->dBinv, c->dMask,
+                                   r64, w[0], w[1], w[5], w[2], w[3], w[4], maxIter, rtol * rtol, iters, relres,
+                                   c->dBatchTicket, s));
     return ef_launch_add(n, xd, w[0], x, s);
 }
 

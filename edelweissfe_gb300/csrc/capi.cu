@@ -292,6 +292,7 @@ void ef_destroy(ef_ctx* c) {
     for (float* p : c->chebD) F(p);
     F(c->dBatchNodePtr);
     F(c->dBatchOrder);
+    for (void* p : c->batchMem) F(p);
     F(c->vcIn);
     F(c->vcOut);
     if (c->vcGraph) cudaGraphExecDestroy(c->vcGraph);

@@ -158,10 +158,11 @@ ef_status ef_mpnn_alpha_combine(int64_t n, const float* Mv, const float* N, cons
 // batch.cu
 int ef_batch_num_tiles();
 void ef_batch_tile_shape(int tile, int* tpb, int* lpr);
-ef_status ef_launch_batched_pcg(int tile, int nSM, int nProb, const int32_t* nodePtr, const int32_t* order,
-                                const int32_t* rowPtr, const int32_t* colIdx, const double* vals, const double* binv,
-                                const uint8_t* mask, const double* b, double* x, double* r, double* z, double* p,
-                                double* q, int maxIter, double rtol2, int* iters, double* rel, cudaStream_t s);
+int ef_batch_cluster_size(int nSM, const std::vector<int>& sizes);
+ef_status ef_launch_batched_pcg(int tile, const BatchPlanDev& pl, int cluster, int nSM, int nProb, const int32_t* rowPtr,
+                                const int32_t* colIdx, const double* bsr, const double* binv, const uint8_t* mask,
+                                const double* b, double* x, double* r, double* r2, double* z, double* p, double* q,
+                                int maxIter, double rtol2, int* iters, double* rel, int* ticket, cudaStream_t s);
 ef_status ef_launch_batch_norms(int nProb, const int32_t* nodePtr, const double* R, const double* F, const double* D,
                                 double* out, cudaStream_t s);
 // fgmres.cu
@@ -565,7 +566,11 @@ struct ef_ctx {
     // batch of independent problems (contiguous node ranges), see ef_batch_setup
     int batchN = 0;
     int32_t *dBatchNodePtr = nullptr, *dBatchOrder = nullptr;
-    int batchTile = 1;  // index into the batched-PCG tile shapes
+    int batchTile = 6;  // index into the batched-PCG tile shapes
+    int batchCluster = 1;                                // CTAs per problem
+    BatchPlanDev batchPlan[3];                           // sliced copies for 1, 4 and 8 lanes per row (one buffer)
+    std::vector<void*> batchMem;                         // their device arrays
+    int* dBatchTicket = nullptr;
     // FGMRES workspace
     float* fgV = nullptr;                // [restart+1][nDof]
     float* fgZ = nullptr;                // [restart][nDof]

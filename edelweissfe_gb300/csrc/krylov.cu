@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "cluster.cuh"
 #include "ef_common.cuh"
 #include "pcg_plan.h"
 
@@ -245,29 +246,6 @@ __device__ __forceinline__ void slot_clear(double* p) {
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %1};\n" ::"l"(p), "l"(kPcgEmpty) : "memory");
 }
 
-// the address of a shared-memory variable of this CTA in CTA `rank` of its cluster
-__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
-    unsigned a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void cluster_store(unsigned a, unsigned long long u, unsigned long long v) {
-    asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};\n" ::"r"(a), "l"(u), "l"(v) : "memory");
-}
-__device__ __forceinline__ float cluster_load(unsigned a, float) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ double cluster_load(unsigned a, double) {
-    double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];\n" : "=d"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
-}
-
 template <typename VT, int TPB>
 struct PcgShared {
     VT red[2][sizeof(VT) == 4 ? TPB / 32 : TPB];
@@ -423,31 +401,6 @@ struct PcgScalars {
     static __device__ bool below(double a, double b) { return a <= b; }
     static __device__ bool below(Sum32 a, Sum32 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo <= b.lo); }
 };
-
-// y += A p of one block as chains of fused multiply-adds (written as a sum of products it is four FP64
-// instructions a row instead of three)
-template <typename VT>
-__device__ __forceinline__ void block_fma(const VT* v, VT p0, VT p1, VT p2, VT& y0, VT& y1, VT& y2) {
-    y0 = fma(v[2], p2, fma(v[1], p1, fma(v[0], p0, y0)));
-    y1 = fma(v[5], p2, fma(v[4], p1, fma(v[3], p0, y1)));
-    y2 = fma(v[8], p2, fma(v[7], p1, fma(v[6], p0, y2)));
-}
-
-// Component c of (y0, y1, y2) summed over the LPR lanes of a row, in the lanes whose top two bits of
-// the group lane are c (c = 3: none).  The first two steps exchange components instead of summing all three in
-// every lane: 3 adds and one per further step against 3 per step.
-template <int LPR, typename VT>
-__device__ __forceinline__ VT row_sum3(int l, VT y0, VT y1, VT y2) {
-    const bool hi = (l & (LPR / 2)) != 0, lo = (l & (LPR / 4)) != 0;
-    VT k0 = hi ? y2 : y0, k1 = hi ? (VT)0 : y1;
-    k0 += __shfl_xor_sync(0xffffffffu, hi ? y0 : y2, LPR / 2);
-    k1 += __shfl_xor_sync(0xffffffffu, hi ? y1 : (VT)0, LPR / 2);
-    VT k = lo ? k1 : k0;
-    k += __shfl_xor_sync(0xffffffffu, lo ? k0 : k1, LPR / 4);
-#pragma unroll
-    for (int o = LPR / 8; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-    return k;
-}
 
 // Block-Jacobi PCG on the free DOFs.  The search direction p_k = z_k + beta_k p_{k-1} is never
 // materialised before the product: each row group gathers z and the previous p of its neighbours and

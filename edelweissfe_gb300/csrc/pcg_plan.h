@@ -1,5 +1,5 @@
-// Host-side plan of the resident PCG kernel (krylov.cu): which rows a CTA keeps, gathers and how its blocks
-// are sliced.
+// Host-side plans of the PCG kernels: the resident PCG (krylov.cu: which rows a CTA keeps and gathers and how
+// its blocks are sliced) and the batched PCG (batch.cu: its sliced copy of the system).
 #pragma once
 
 #include <stddef.h>
@@ -24,3 +24,17 @@ struct PcgResidentPlan {
 
 void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPtr, const int32_t* colIdx,
                           PcgResidentPlan& plan);
+
+// The batched PCG's sliced copy for one number of lanes per block row: device arrays
+struct BatchPlanDev {
+    int nGroups = 0;                       // groups of 32 / lanes rows, none across two problems
+    const int32_t *nodePtr = nullptr;      // [problems + 1]
+    const int32_t *order = nullptr;        // [problems] by decreasing size
+    const int32_t *groupBase = nullptr;    // [problems] a problem's first entry of groupPtr
+    const int32_t *groupPtr = nullptr;     // per problem [groups + 1] first step of each group
+    const int32_t *groupRow = nullptr;     // [groups] first row
+    const int32_t *groupEnd = nullptr;     // [groups] the problem's end row
+    const int32_t *groupStep = nullptr;    // [groups][2] first and last step
+    double* vals = nullptr;                // [steps][9][32]
+    int32_t* col = nullptr;                // [steps][32]
+};

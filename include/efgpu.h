@@ -289,12 +289,14 @@ ef_status ef_set_group_props(ef_ctx* ctx, int groupId, const double* table, int 
 /* Declares the problems: problem p owns the nodes [nodePtr[p], nodePtr[p+1]) (host int32
  * [nProb+1], covering all nodes); no 3x3 block may couple two problems.  Needs EF_OPT_KE_FP64. */
 ef_status ef_batch_setup(ef_ctx* ctx, int nProb, const int32_t* nodePtr);
-/* Tile shapes of the batched PCG: tile t in [0, ef_batch_tile_count()) runs threadsPerCta threads
- * per problem with lanesPerRow lanes per 3x3 block row in the matrix products. */
+/* Tile shapes of the batched PCG: tile t in [0, ef_batch_tile_count()) runs CTAs of threadsPerCta
+ * threads with lanesPerRow lanes per 3x3 block row in the matrix products.  A problem is solved by a
+ * cluster of 1, 2, 4 or 8 CTAs, chosen from the problems' sizes by ef_batch_setup. */
 int ef_batch_tile_count(void);
 ef_status ef_batch_tile_info(int tile, int* threadsPerCta, int* lanesPerRow);
 ef_status ef_batch_set_tile(ef_ctx* ctx, int tile);
-/* Solves K x = b problem by problem in one persistent launch (block-Jacobi PCG, FP64): Dirichlet
+/* Solves K x = b problem by problem in one persistent launch (block-Jacobi PCG, FP64; a launch before it
+ * brings the blocks into the kernel's order): Dirichlet
  * DOFs take b, each problem stops at |r| <= rtol |b_p| (its lifted right-hand side) or maxIter.
  * b, x device FP64 [nDof]; iters (device int32 [nProb]) and relres (device FP64 [nProb]) receive
  * each problem's iteration count and final relative residual (NaN on breakdown).  Does not
