@@ -12,41 +12,78 @@
 // bit-reproducible run to run.
 
 #include "ef_common.cuh"
+#include "reduce.cuh"
+
+#include <algorithm>
 
 namespace ef {
 
-// P[d0+c] = sum_k Pe[src_k + c], F likewise with |.|; one thread per node (DOF triplet)
-__global__ void condense_kernel(int64_t nNodes, const int32_t* __restrict__ nodeDof, const int64_t* __restrict__ ptr,
-                                const int64_t* __restrict__ src, const float* __restrict__ w,
-                                const double* __restrict__ Pe, double* __restrict__ P, double* __restrict__ F) {
-    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= nNodes) return;
-    double p0 = 0.0, p1 = 0.0, p2 = 0.0, f0 = 0.0, f1 = 0.0, f2 = 0.0;
-    for (int64_t k = ptr[m]; k < ptr[m + 1]; ++k) {
-        const double* pe = Pe + src[k];
-        double a = pe[0], b = pe[1], c = pe[2];
-        if (w) {  // tied node: weighted share of the slave's element vectors
-            const double wk = w[k];
-            a *= wk;
-            b *= wk;
-            c *= wk;
+// Sum over the sources of one DOF (component c of node m) in source order, and of their absolute values; the
+// loads of eight sources are in flight together (an interior hex8 node has eight), where one source after the
+// other cost eight trips to memory
+template <bool ABS>
+__device__ __forceinline__ void condense_dof(int64_t k0, int64_t k1, int c, const int64_t* __restrict__ src,
+                                             const float* __restrict__ w, const double* __restrict__ Pe, double& p,
+                                             double& f) {
+    p = f = 0.0;
+    for (int64_t k = k0; k < k1; k += 8) {
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (k + j < k1) {
+                v[j] = Pe[src[k + j] + c];
+                if (w) v[j] *= (double)w[k + j];  // tied node: weighted share of the slave's element vectors
+            }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (k + j < k1) {
+                p += v[j];
+                if (ABS) f += fabs(v[j]);
+            }
+    }
+}
+
+// P[d] = sum_k Pe[src_k + c], F likewise with |.| (F may be null); a thread per DOF
+template <bool ABS>
+__global__ void __launch_bounds__(kRedThreads) condense_kernel(int64_t nNodes, const int32_t* __restrict__ nodeDof,
+                                                               const int64_t* __restrict__ ptr,
+                                                               const int64_t* __restrict__ src,
+                                                               const float* __restrict__ w, const double* __restrict__ Pe,
+                                                               double* __restrict__ P, double* __restrict__ F) {
+    const int64_t t = (int64_t)blockIdx.x * kRedThreads + threadIdx.x;
+    if (t >= 3 * nNodes) return;
+    const int64_t m = t / 3;
+    const int c = (int)(t - 3 * m);
+    double p, f;
+    condense_dof<ABS>(ptr[m], ptr[m + 1], c, src, w, Pe, p, f);
+    const int d = nodeDof[m] + c;
+    P[d] = p;
+    if (ABS) F[d] = f;
+}
+
+// r = b - (condensed ye) on free DOFs, 0 on masked ones (b may be null: r = condensed ye) and, with out,
+// *out = sum r^2: the refinement residual from its element vectors in one pass
+__global__ void __launch_bounds__(kRedThreads) condense_residual_kernel(
+    int64_t nNodes, const int32_t* __restrict__ nodeDof, const int64_t* __restrict__ ptr,
+    const int64_t* __restrict__ src, const float* __restrict__ w, const double* __restrict__ ye,
+    const double* __restrict__ b, const uint8_t* __restrict__ mask, double* __restrict__ r, double* part,
+    unsigned* ticket, double* out) {
+    double v[1] = {0.0};
+    for (int64_t t = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; t < 3 * nNodes;
+         t += (int64_t)gridDim.x * kRedThreads) {
+        const int64_t m = t / 3;
+        const int c = (int)(t - 3 * m);
+        const int d = nodeDof[m] + c;
+        double y = 0.0, f;
+        if (!mask[d]) {
+            condense_dof<false>(ptr[m], ptr[m + 1], c, src, w, ye, y, f);
+            if (b) y = b[d] - y;
         }
-        p0 += a;
-        p1 += b;
-        p2 += c;
-        f0 += fabs(a);
-        f1 += fabs(b);
-        f2 += fabs(c);
+        r[d] = y;
+        v[0] += y * y;
     }
-    const int d = nodeDof[m];
-    P[d] = p0;
-    P[d + 1] = p1;
-    P[d + 2] = p2;
-    if (F) {
-        F[d] = f0;
-        F[d + 1] = f1;
-        F[d + 2] = f2;
-    }
+    if (!out) return;
+    if (grid_reduce<1, 0u>(v, part, ticket)) *out = v[0];
 }
 
 // adds the condensed element vectors into V (V[d] += sum), used for body forces
@@ -184,104 +221,51 @@ __global__ void bj_setup_kernel(int64_t nNodes, const int64_t* __restrict__ diag
     o[8] = (KT)((A[0][0] * A[1][1] - A[0][1] * A[1][0]) * id);
 }
 
-// deterministic norms: per-block partials in a fixed order, then one block reduces them
-__global__ void norms_partial_kernel(int64_t n, const double* __restrict__ R, const double* __restrict__ F,
-                                     const double* __restrict__ D, double* __restrict__ part) {
-    __shared__ double s0[256], s1[256], s2[256];
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (R) a = fmax(a, fabs(R[i]));
-        if (F) b += fabs(F[i]);
-        if (D) c = fmax(c, fabs(D[i]));
+// out = {max |R|, sum |F|, max |D|} (each may be null -> 0)
+__global__ void __launch_bounds__(kRedThreads) norms_kernel(int64_t n, const double* __restrict__ R,
+                                                            const double* __restrict__ F, const double* __restrict__ D,
+                                                            double* part, unsigned* ticket, double* out) {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads) {
+        if (R) v[0] = fmax(v[0], fabs(R[i]));
+        if (F) v[1] += fabs(F[i]);
+        if (D) v[2] = fmax(v[2], fabs(D[i]));
     }
-    s0[threadIdx.x] = a;
-    s1[threadIdx.x] = b;
-    s2[threadIdx.x] = c;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-            s1[threadIdx.x] += s1[threadIdx.x + w];
-            s2[threadIdx.x] = fmax(s2[threadIdx.x], s2[threadIdx.x + w]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x + 0] = s0[0];
-        part[3 * blockIdx.x + 1] = s1[0];
-        part[3 * blockIdx.x + 2] = s2[0];
+    if (grid_reduce<3, 5u>(v, part, ticket)) {
+        out[0] = v[0];
+        out[1] = v[1];
+        out[2] = v[2];
     }
 }
 
-__global__ void norms_final_kernel(int nPart, const double* __restrict__ part, double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = 0; i < nPart; ++i) {
-        a = fmax(a, part[3 * i]);
-        b += part[3 * i + 1];
-        c = fmax(c, part[3 * i + 2]);
-    }
-    out[0] = a;
-    out[1] = b;
-    out[2] = c;
-}
-
-// R = P + PExt with the Dirichlet rows set to 0 (dir[i] != 0), and the partial norms of the
-// convergence check: max |R|, sum |F|, max |ddU| (solvers/nonlinearimplicitstatic.py:418-436,
-// :625-725)
-__global__ void newton_residual_kernel(int64_t n, const double* __restrict__ P, const double* __restrict__ PExt,
-                                       const uint8_t* __restrict__ dir, const double* __restrict__ F,
-                                       const double* __restrict__ D, double* __restrict__ R,
-                                       double* __restrict__ part) {
-    __shared__ double s0[256], s1[256], s2[256];
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+// R = P + PExt with the Dirichlet rows set to 0 (dir[i] != 0), the norms of the convergence check (max |R|,
+// sum |F|, max |ddU|; solvers/nonlinearimplicitstatic.py:418-436, :625-725) and, by the thread that gets
+// them, the reference's test for the displacement field (:656-682, computeSpatialAveragedFluxes :771-792):
+// out = {converged, nGrew, fluxResidual, fieldCorrection, spatialAveragedFlux}
+__global__ void __launch_bounds__(kRedThreads) newton_check_kernel(int64_t n, const double* __restrict__ P,
+                                                                   const double* __restrict__ PExt,
+                                                                   const uint8_t* __restrict__ dir,
+                                                                   const double* __restrict__ F,
+                                                                   const double* __restrict__ D, double* __restrict__ R,
+                                                                   double* part, unsigned* ticket, NewtonTest q,
+                                                                   double* out) {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads) {
         const double r = dir[i] ? 0.0 : (PExt ? P[i] + PExt[i] : P[i]);
         R[i] = r;
-        a = fmax(a, fabs(r));
-        b += fabs(F[i]);
-        if (D) c = fmax(c, fabs(D[i]));
+        v[0] = fmax(v[0], fabs(r));
+        v[1] += fabs(F[i]);
+        if (D) v[2] = fmax(v[2], fabs(D[i]));
     }
-    s0[threadIdx.x] = a;
-    s1[threadIdx.x] = b;
-    s2[threadIdx.x] = c;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-            s1[threadIdx.x] += s1[threadIdx.x + w];
-            s2[threadIdx.x] = fmax(s2[threadIdx.x], s2[threadIdx.x + w]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x + 0] = s0[0];
-        part[3 * blockIdx.x + 1] = s1[0];
-        part[3 * blockIdx.x + 2] = s2[0];
-    }
-}
-
-// The reference's convergence test for the displacement field (solvers/nonlinearimplicitstatic.py
-// :656-682, computeSpatialAveragedFluxes :771-792), decided on the device from the partial norms:
-// q = {fluxTol, fluxTolAlt, corrTol, fluxFloor, nAccFluxes, prevResidual, iteration, nGrew, hasDdU}
-// out = {converged, nGrew, fluxResidual, fieldCorrection, spatialAveragedFlux}
-__global__ void newton_decide_kernel(int nPart, const double* __restrict__ part, const double* __restrict__ q,
-                                     double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = 0; i < nPart; ++i) {
-        a = fmax(a, part[3 * i]);
-        b += part[3 * i + 1];
-        c = fmax(c, part[3 * i + 2]);
-    }
-    const double avg = fmax(1e-10, b / q[4]);
-    const double tol = q[6] < 15.0 ? q[0] : q[1];
-    const double corr = q[8] != 0.0 ? c : 0.0;
-    const bool convCorr = corr < q[2];
-    const bool convFlux = a <= fmax(tol * avg, q[3]);
+    if (!grid_reduce<3, 5u>(v, part, ticket)) return;
+    const double avg = fmax(1e-10, v[1] / q.nAccFluxes);
+    const double tol = q.iteration < 15 ? q.fluxTol : q.fluxTolAlt;
+    const double corr = D ? v[2] : 0.0;
+    const bool convCorr = corr < q.corrTol;
+    const bool convFlux = v[0] <= fmax(tol * avg, q.fluxFloor);
     out[0] = (convCorr && convFlux) ? 1.0 : 0.0;
-    out[1] = q[7] + (a > q[5] ? 1.0 : 0.0);
-    out[2] = a;
+    out[1] = q.nGrew + (v[0] > q.prevResidual ? 1.0 : 0.0);
+    out[2] = v[0];
     out[3] = corr;
     out[4] = avg;
 }
@@ -317,7 +301,24 @@ static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 ef_status ef_launch_condense(int64_t nNodes, const int32_t* nodeDof, const int64_t* ptr, const int64_t* src,
                              const float* w, const double* Pe, double* P, double* F, cudaStream_t s) {
     if (nNodes == 0) return EF_OK;
-    condense_kernel<<<nblk(nNodes, 256), 256, 0, ef::counted(s)>>>(nNodes, nodeDof, ptr, src, w, Pe, P, F);
+    if (F)
+        condense_kernel<true><<<nblk(3 * nNodes, kRedThreads), kRedThreads, 0, ef::counted(s)>>>(nNodes, nodeDof, ptr, src,
+                                                                                                w, Pe, P, F);
+    else
+        condense_kernel<false><<<nblk(3 * nNodes, kRedThreads), kRedThreads, 0, ef::counted(s)>>>(nNodes, nodeDof, ptr, src,
+                                                                                                 w, Pe, P, F);
+    EF_CUDA(cudaGetLastError());
+    return EF_OK;
+}
+
+// nPart: the number of CTAs' results `part` has room for
+ef_status ef_launch_condense_residual(int64_t nNodes, const int32_t* nodeDof, const int64_t* ptr, const int64_t* src,
+                                      const float* w, const double* ye, const double* b, const uint8_t* mask, double* r,
+                                      double* part, int nPart, unsigned* ticket, double* out, cudaStream_t s) {
+    if (nNodes == 0) return EF_OK;
+    const int grid = std::min(nblk(3 * nNodes, kRedThreads), nPart);
+    condense_residual_kernel<<<grid, kRedThreads, 0, ef::counted(s)>>>(nNodes, nodeDof, ptr, src, w, ye, b, mask, r, part,
+                                                                      ticket, out);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }
@@ -383,34 +384,18 @@ ef_status ef_launch_bj_setup(int64_t nNodes, const int64_t* diagPos, const int32
     return EF_OK;
 }
 
-__global__ void residual_from_kernel(int64_t n, const double* __restrict__ b, const double* __restrict__ y,
-                                     const uint8_t* __restrict__ mask, double* __restrict__ r) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    r[i] = (mask && mask[i]) ? 0.0 : (b ? b[i] - y[i] : y[i]);
-}
-
-ef_status ef_launch_residual_from(int64_t n, const double* b, const double* y, const uint8_t* mask, double* r,
-                                  cudaStream_t s) {
-    if (n == 0) return EF_OK;
-    residual_from_kernel<<<nblk(n, 256), 256, 0, ef::counted(s)>>>(n, b, y, mask, r);
-    EF_CUDA(cudaGetLastError());
-    return EF_OK;
-}
-
 ef_status ef_launch_norms(int64_t n, const double* R, const double* F, const double* D, double* part, int nPart,
-                          double* out, cudaStream_t s) {
-    norms_partial_kernel<<<nPart, 256, 0, ef::counted(s)>>>(n, R, F, D, part);
-    norms_final_kernel<<<1, 32, 0, ef::counted(s)>>>(nPart, part, out);
+                          unsigned* ticket, double* out, cudaStream_t s) {
+    norms_kernel<<<reduce_grid(n, nPart), kRedThreads, 0, ef::counted(s)>>>(n, R, F, D, part, ticket, out);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }
 
 ef_status ef_launch_newton_check(int64_t n, const double* P, const double* PExt, const uint8_t* dir, const double* F,
-                                 const double* D, double* R, double* part, int nPart, const double* q, double* out,
-                                 cudaStream_t s) {
-    newton_residual_kernel<<<nPart, 256, 0, ef::counted(s)>>>(n, P, PExt, dir, F, D, R, part);
-    newton_decide_kernel<<<1, 32, 0, ef::counted(s)>>>(nPart, part, q, out);
+                                 const double* D, double* R, double* part, int nPart, unsigned* ticket,
+                                 const NewtonTest& q, double* out, cudaStream_t s) {
+    newton_check_kernel<<<reduce_grid(n, nPart), kRedThreads, 0, ef::counted(s)>>>(n, P, PExt, dir, F, D, R, part, ticket,
+                                                                                 q, out);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }

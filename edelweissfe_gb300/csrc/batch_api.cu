@@ -142,7 +142,7 @@ static ef_status batch_solve(ef_ctx* c, int tile, double rtol, int maxIter, cons
     double* r64 = c->w64[2];
     // Dirichlet DOFs take b; the free part solves K_ff x_f = b_f - K_fd x_d per problem
     EF_CHECK(ef_launch_masked_copy(n, b, c->dMask, 1, 1.0, xd, 1, s));
-    EF_CHECK(residual64(c, xd, b, r64, s));
+    EF_CHECK(residual64(c, xd, b, r64, nullptr, s));
     double* w[6];
     for (int i = 0; i < 6; ++i) w[i] = (double*)c->w64k[1 + i];
     int tpb = 0, lpr = 0;

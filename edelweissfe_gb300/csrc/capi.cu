@@ -230,7 +230,6 @@ void ef_destroy(ef_ctx* c) {
     F(c->dFlags);
     F(c->dDirIdx);
     F(c->dDirMask);
-    F(c->dNewton);
     F(c->dSellOff);
     F(c->dSellPerm);
     F(c->dSellCol);
@@ -271,13 +270,13 @@ void ef_destroy(ef_ctx* c) {
     F(c->dCsrPerm);
     F(c->dKvijTmp);
     F(c->dPart);
-    F(c->dRed);
+    F(c->dTicket);
+    if (c->hRes) cudaFreeHost(c->hRes);
     F(c->dPcgSlots);
     F(c->dPcgHaloPtr);
     F(c->dPcgHaloIdx);
     F(c->dPcgGroupPtr);
     F(c->dPcgLcol);
-    F(c->dPcgRes);
     for (auto* p : c->w32) F(p);
     for (auto* p : c->w64) F(p);
     for (auto* p : c->w64k) F(p);
@@ -912,13 +911,15 @@ ef_status ef_finalize(ef_ctx* c, int options) {
     }
 
     // reduction and Krylov workspaces
-    c->nPart = 2 * c->nSM;
+    c->nPart = 16 * c->nSM;
     c->dPart = dalloc<double>(4 * c->nPart, &st);
-    c->dRed = dalloc<double>(16, &st);
-    if (!c->dPart || !c->dRed) return st;
+    c->dTicket = dalloc<unsigned>(1, &st);
+    if (!c->dPart || !c->dTicket) return st;
+    EF_CUDA(cudaMemset(c->dTicket, 0, sizeof(unsigned)));
+    EF_CUDA(cudaHostAlloc((void**)&c->hRes, sizeof(HostResults), cudaHostAllocMapped));
+    EF_CUDA(cudaHostGetDevicePointer((void**)&c->hResDev, c->hRes, 0));
     c->dPcgSlots = dalloc<double>(ef_pcg_slot_bytes(ef_pcg_slot_sets()) / sizeof(double), &st);
-    c->dPcgRes = dalloc<char>(ef_pcg_result_bytes(), &st);
-    if (!c->dPcgSlots || !c->dPcgRes) return st;
+    if (!c->dPcgSlots) return st;
     for (int i = 0; i < 7; ++i) {
         c->w32[i] = dalloc<float>(c->nDof, &st);
         if (!c->w32[i]) return st;
@@ -1038,14 +1039,14 @@ ef_status ef_compute_elements(ef_ctx* c, const double* U_np, const double* dU, c
 
 ef_status ef_element_status(ef_ctx* c, void* stream, double* pNewDT) {
     EF_REQUIRE_FINALIZED(c);
-    int hf[2] = {0, 0};
-    EF_CUDA(cudaMemcpyAsync(hf, c->dFlags, sizeof(hf), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    int* hf = c->hRes->flags;
+    EF_CUDA(cudaMemcpyAsync(hf, c->dFlags, sizeof(c->hRes->flags), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     EF_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     const int f = hf[0];
-    float req = EF_PNEWDT_NONE;
+    const float none = EF_PNEWDT_NONE;
+    float req = none;
     memcpy(&req, &hf[1], sizeof(float));
-    {
-        const float none = EF_PNEWDT_NONE;
+    if (f != 0 || !(req == none)) {
         int reset[2] = {0, 0};
         memcpy(&reset[1], &none, sizeof(float));
         EF_CUDA(cudaMemcpy(c->dFlags, reset, sizeof(reset), cudaMemcpyHostToDevice));

@@ -19,10 +19,8 @@
 #include "pcg_plan.h"
 
 // krylov.cu
-int ef_krylov_block_threads();
 int ef_pcg_slot_sets();
 size_t ef_pcg_slot_bytes(int sets);
-size_t ef_pcg_result_bytes();
 ef_status ef_launch_bsr_residual(int nNodes, const int32_t* rowPtr, const int32_t* colIdx, const void* vals,
                                  int mDouble, const double* x, const double* b, const uint8_t* mask, double* y,
                                  int nSM, cudaStream_t s);
@@ -35,8 +33,12 @@ ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes,
                                  const int32_t* groupPtr, size_t smem, const void* vals, const void* binv,
                                  const uint8_t* mask, const void* b, void* x, void* z, double* slots, void* res,
                                  int maxIter, double rtol2, int* flags, cudaStream_t s);
-ef_status ef_launch_dot(int64_t n, const double* a, const double* b, double* part, int nPart, double* out,
-                        cudaStream_t s);
+ef_status ef_launch_dot(int64_t n, const double* a, const double* b, double* part, int nPart, unsigned* ticket,
+                        double* out, cudaStream_t s);
+ef_status ef_launch_solve_begin(int64_t n, const double* b, const uint8_t* mask, double* xd, double* xf, double* r,
+                                double* part, int nPart, unsigned* ticket, double* out, cudaStream_t s);
+ef_status ef_launch_refine_update(int64_t n, double a, const void* d, int dDouble, const double* xd, double* xf,
+                                  double* sum, cudaStream_t s);
 ef_status ef_launch_masked_copy(int64_t n, const double* src, const uint8_t* mask, int keepMasked, double scale,
                                 void* dst, int dstDouble, cudaStream_t s);
 ef_status ef_launch_axpy(int64_t n, double a, const void* xs, int xDouble, double* y, cudaStream_t s);
@@ -185,8 +187,8 @@ ef_status ef_launch_spmv_f32_staged(int nSM, int cap, int nN, const int32_t* row
 ef_status ef_launch_combine(int64_t n, int nv, const float* Z, int64_t ldz, const double* y, float* x, cudaStream_t s);
 ef_status ef_launch_sub(int64_t n, const float* b, const float* y, float* r, cudaStream_t s);
 ef_status ef_launch_newton_check(int64_t n, const double* P, const double* PExt, const uint8_t* dir, const double* F,
-                                 const double* D, double* R, double* part, int nPart, const double* q, double* out,
-                                 cudaStream_t s);
+                                 const double* D, double* R, double* part, int nPart, unsigned* ticket,
+                                 const ef::NewtonTest& q, double* out, cudaStream_t s);
 ef_status ef_launch_newton_first(int64_t n, const double* P, const double* PExt, int64_t nDir, const int64_t* dofs,
                                  const double* values, double* R, cudaStream_t s);
 ef_status ef_launch_sell_refresh(int64_t nE, const int32_t* src, const float* bsr, float* v9, void* v8, void* v1,
@@ -245,6 +247,12 @@ struct PcgResultHost {
     int status;
     double rr;
     double bb;
+};
+
+struct HostResults {
+    double red[8];   // reductions
+    PcgResultHost pcg;
+    int flags[2];    // copy of the context's device flags
 };
 
 struct HostGroup {
@@ -408,7 +416,6 @@ struct ef_ctx {
     int64_t nDir = 0;
     int64_t* dDirIdx = nullptr;
     uint8_t* dDirMask = nullptr;
-    double* dNewton = nullptr;  // [16]: decision inputs (9) and outputs (5) of ef_newton_residual
     // scalar CSR (reference layout)
     bool scalar = false;
     int64_t nVIJ = 0, nnz = 0;
@@ -421,7 +428,10 @@ struct ef_ctx {
     // reductions / Krylov workspace
     double* dPart = nullptr;
     int nPart = 0;
-    double* dRed = nullptr;  // small result buffer
+    unsigned* dTicket = nullptr;  // last-CTA counter of the reductions (0 between launches)
+    // results that the host reads after a synchronisation, written by the kernels: mapped pinned memory
+    HostResults* hRes = nullptr;
+    HostResults* hResDev = nullptr;
     double* dPcgSlots = nullptr;  // reduction slots of the persistent PCG
     // resident PCG (ef_pcg_resident_plan), made at the context's first PCG solve; the system has one
     // precision, so one plan: 0 bytes of shared memory: the streaming kernel
@@ -430,7 +440,6 @@ struct ef_ctx {
     PcgShape pcgShape;
     int32_t *dPcgHaloPtr = nullptr, *dPcgHaloIdx = nullptr, *dPcgGroupPtr = nullptr;
     uint16_t* dPcgLcol = nullptr;
-    void* dPcgRes = nullptr;
     void* w32[7] = {};  // FP32 Krylov vectors: b, x, r, z, p (two buffers), q
     double* w64[5] = {};  // FP64: xd, xf, r64, tmp, y
     // exact refinement: FP64 Gauss-point tangents per group and an element-vector buffer
@@ -598,7 +607,7 @@ struct ef_ctx {
 
 // ---- functions of one host unit called from another ----------------------------------------
 // system.cu
-ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, cudaStream_t s);
+ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, double* rr, cudaStream_t s);
 ef_status dot_host(ef_ctx* c, const double* a, const double* b, double* out, cudaStream_t s);
 ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol, PcgResultHost* out,
                   ef_solve_info* prof, cudaStream_t s);

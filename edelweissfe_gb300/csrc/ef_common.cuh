@@ -115,6 +115,12 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 #endif
 
+// Inputs of the Newton check (ef_newton_residual)
+struct NewtonTest {
+    double fluxTol, fluxTolAlt, corrTol, fluxFloor, nAccFluxes, prevResidual;
+    int iteration, nGrew;
+};
+
 // One phase of the multigrid cycle below a level, run by coarse_cycle_kernel (amg.cu) with a
 // cluster barrier after each phase.  All coarse nodes carry 6 DOFs.
 enum CoarseOpType {
@@ -182,7 +188,8 @@ ef_status ef_launch_bsr_scatter(int64_t nBlocks, const int64_t* seg, const int64
                                 const void* Kblk, int kDouble, void* vals, cudaStream_t s);
 ef_status ef_launch_bj_setup(int64_t nNodes, const int64_t* diagPos, const int32_t* nodeDof, const uint8_t* mask,
                              const void* vals, int kDouble, void* inv, int* flags, cudaStream_t s);
-ef_status ef_launch_residual_from(int64_t n, const double* b, const double* y, const uint8_t* mask, double* r,
-                                  cudaStream_t s);
+ef_status ef_launch_condense_residual(int64_t nNodes, const int32_t* nodeDof, const int64_t* ptr, const int64_t* src,
+                                      const float* w, const double* ye, const double* b, const uint8_t* mask, double* r,
+                                      double* part, int nPart, unsigned* ticket, double* out, cudaStream_t s);
 ef_status ef_launch_norms(int64_t n, const double* R, const double* F, const double* D, double* part, int nPart,
-                          double* out, cudaStream_t s);
+                          unsigned* ticket, double* out, cudaStream_t s);

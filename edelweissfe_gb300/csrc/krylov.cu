@@ -16,45 +16,13 @@
 #include "cluster.cuh"
 #include "ef_common.cuh"
 #include "pcg_plan.h"
+#include "reduce.cuh"
 
 namespace ef {
 
 constexpr int kKB = 512;         // threads per CTA of the Krylov kernels
 constexpr int kRowLanes = 8;     // lanes per block row in the SpMV
 constexpr int kBatch = 4;        // blocks per lane whose loads are issued together
-
-// FP64 is a narrow pipe on this GPU (2 lanes per SM and cycle): per-thread partial sums and the
-// warp trees run in the vector type AT (FP32 for the FP32 solve), the CTA's warp sums and the
-// sum over CTAs in FP64, all in a fixed order.
-
-// CTA sum of NV values per thread, returned in FP64 to every thread
-template <typename AT, int NV>
-__device__ __forceinline__ void block_sum(AT (&v)[NV], double (&out)[NV]) {
-    constexpr int NW = kKB / 32;
-    __shared__ AT red[NV][NW];
-    __shared__ double res[NV];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < NV; ++j) red[j][w] = v[j];
-    }
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < NW; ++q) t += (double)red[threadIdx.x][q];
-        res[threadIdx.x] = t;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NV; ++j) out[j] = res[j];
-    __syncthreads();
-}
 
 // y_row = A_row x for the block row `m`, lanes l = 0..7 of a row group; returns partial sums
 // CG = true loads x through L2 only (x was written by other CTAs of a persistent kernel)
@@ -752,22 +720,49 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
     }
 }
 
-// deterministic dot products: part[c*2+{0,1}] then a final pass
-__global__ void __launch_bounds__(kKB) dot2_partial_kernel(int64_t n, const double* __restrict__ a,
-                                                           const double* __restrict__ b, double* __restrict__ part) {
+// *out = a . b
+__global__ void __launch_bounds__(kRedThreads) dot_kernel(int64_t n, const double* __restrict__ a,
+                                                          const double* __restrict__ b, double* part, unsigned* ticket,
+                                                          double* out) {
     double v[1] = {0.0};
-    for (int64_t i = (int64_t)blockIdx.x * kKB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kKB)
+    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
         v[0] += a[i] * b[i];
-    double o[1];
-    block_sum<double, 1>(v, o);
-    if (threadIdx.x == 0) part[blockIdx.x] = o[0];
+    if (grid_reduce<1, 0u>(v, part, ticket)) *out = v[0];
 }
 
-__global__ void sum_final_kernel(int n, const double* __restrict__ part, double* __restrict__ out) {
-    if (threadIdx.x || blockIdx.x) return;
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
+// The start of a solve in one pass: xd = b on masked DOFs, r = b on free ones, xf = 0;
+// out = {b.b, xd.xd, r.r}
+__global__ void __launch_bounds__(kRedThreads) solve_begin_kernel(int64_t n, const double* __restrict__ b,
+                                                                  const uint8_t* __restrict__ mask,
+                                                                  double* __restrict__ xd, double* __restrict__ xf,
+                                                                  double* __restrict__ r, double* part, unsigned* ticket,
+                                                                  double* out) {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads) {
+        const double bi = b[i], d = mask[i] ? bi : 0.0, f = mask[i] ? 0.0 : bi;
+        xd[i] = d;
+        xf[i] = 0.0;
+        r[i] = f;
+        v[0] += bi * bi;
+        v[1] += d * d;
+        v[2] += f * f;
+    }
+    if (grid_reduce<3, 0u>(v, part, ticket)) {
+        out[0] = v[0];
+        out[1] = v[1];
+        out[2] = v[2];
+    }
+}
+
+// xf += a d, sum = xd + xf: the refinement's new iterate and the point of its residual
+template <typename T>
+__global__ void refine_update_kernel(int64_t n, double a, const T* __restrict__ d, const double* __restrict__ xd,
+                                     double* __restrict__ xf, double* __restrict__ sum) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double f = xf[i] + a * (double)d[i];
+    xf[i] = f;
+    sum[i] = xd[i] + f;
 }
 
 // small vector kernels
@@ -807,10 +802,8 @@ static int pcg_lanes(int rows, int tpb, int vDouble) {
     return lpr;
 }
 
-int ef_krylov_block_threads() { return kKB; }
 int ef_pcg_slot_sets() { return kPcgMaxCopies; }
 size_t ef_pcg_slot_bytes(int sets) { return sets * kPcgSlotBytes; }
-size_t ef_pcg_result_bytes() { return sizeof(PcgResult); }
 
 ef_status ef_launch_bsr_residual(int nNodes, const int32_t* rowPtr, const int32_t* colIdx, const void* vals,
                                  int mDouble, const double* x, const double* b, const uint8_t* mask, double* y,
@@ -1006,10 +999,28 @@ ef_status ef_launch_pcg(int vDouble, int nSM, int nNodes, const int32_t* rowPtr,
     return EF_OK;
 }
 
-ef_status ef_launch_dot(int64_t n, const double* a, const double* b, double* part, int nPart, double* out,
-                        cudaStream_t s) {
-    dot2_partial_kernel<<<nPart, kKB, 0, ef::counted(s)>>>(n, a, b, part);
-    sum_final_kernel<<<1, 32, 0, ef::counted(s)>>>(nPart, part, out);
+ef_status ef_launch_dot(int64_t n, const double* a, const double* b, double* part, int nPart, unsigned* ticket,
+                        double* out, cudaStream_t s) {
+    dot_kernel<<<reduce_grid(n, nPart), kRedThreads, 0, ef::counted(s)>>>(n, a, b, part, ticket, out);
+    EF_CUDA(cudaGetLastError());
+    return EF_OK;
+}
+
+ef_status ef_launch_solve_begin(int64_t n, const double* b, const uint8_t* mask, double* xd, double* xf, double* r,
+                                double* part, int nPart, unsigned* ticket, double* out, cudaStream_t s) {
+    solve_begin_kernel<<<reduce_grid(n, nPart), kRedThreads, 0, ef::counted(s)>>>(n, b, mask, xd, xf, r, part, ticket,
+                                                                                out);
+    EF_CUDA(cudaGetLastError());
+    return EF_OK;
+}
+
+ef_status ef_launch_refine_update(int64_t n, double a, const void* d, int dDouble, const double* xd, double* xf,
+                                  double* sum, cudaStream_t s) {
+    if (n == 0) return EF_OK;
+    if (dDouble)
+        refine_update_kernel<double><<<nb(n, 256), 256, 0, ef::counted(s)>>>(n, a, (const double*)d, xd, xf, sum);
+    else
+        refine_update_kernel<float><<<nb(n, 256), 256, 0, ef::counted(s)>>>(n, a, (const float*)d, xd, xf, sum);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }

@@ -326,19 +326,13 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
     ef_solve_info inf;
     memset(&inf, 0, sizeof(inf));
     inf.status = EF_OK;
-    double bb = 0.0;
-    EF_CHECK(dot_host(c, b, b, &bb, s));
     // Dirichlet part: x_d = b on Dirichlet DOFs; lifted RHS b~ = b_f - K_fd x_d (when x_d = 0, as in
     // every Newton system after an increment's first, b~ is b on the free DOFs: the same bits
     // without the operator application)
-    EF_CHECK(ef_launch_masked_copy(n, b, c->dMask, 1, 1.0, xd, 1, s));
-    double dd = 0.0;
-    EF_CHECK(dot_host(c, xd, xd, &dd, s));
-    if (dd == 0.0)
-        EF_CHECK(ef_launch_masked_copy(n, b, c->dMask, 0, 1.0, r64, 1, s));
-    else
-        EF_CHECK(residual64(c, xd, b, r64, s));
-    EF_CUDA(cudaMemsetAsync(xf, 0, sizeof(double) * n, s));
+    EF_CHECK(ef_launch_solve_begin(n, b, c->dMask, xd, xf, r64, c->dPart, c->nPart, c->dTicket, c->hResDev->red, s));
+    EF_CUDA(cudaStreamSynchronize(s));
+    const double bb = c->hRes->red[0], dd = c->hRes->red[1];
+    double rr = c->hRes->red[2];
     if (!(bb > 0.0)) {
         EF_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
         inf.relResidual = 0.0;
@@ -346,8 +340,7 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
         return EF_OK;
     }
     const double bnorm = sqrt(bb);
-    double rr = 0.0;
-    EF_CHECK(dot_host(c, r64, r64, &rr, s));
+    if (dd != 0.0) EF_CHECK(residual64(c, xd, b, r64, &rr, s));
     int total = 0;
     ef_status result = EF_OK;
     if (!o->mixed) {
@@ -419,11 +412,9 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
                 break;
             }
             if (pr.iterations == 0) break;  // no progress possible
-            EF_CHECK(ef_launch_axpy(n, rn, wv[1], vd, xf, s));
             // r64 = b~ - K x_f  (FP64 accumulation); b~ = b - K x_d on free rows
-            EF_CHECK(ef_launch_add(n, xd, xf, tmp, s));
-            EF_CHECK(residual64(c, tmp, b, r64, s));
-            EF_CHECK(dot_host(c, r64, r64, &rr, s));
+            EF_CHECK(ef_launch_refine_update(n, rn, wv[1], vd, xd, xf, tmp, s));
+            EF_CHECK(residual64(c, tmp, b, r64, &rr, s));
         }
     }
     EF_CHECK(ef_launch_add(n, xd, xf, x, s));
@@ -432,8 +423,7 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
     // leaves r64 = b - K (x_d + x_f) of this very x (every exit follows a residual of the current
     // x_f), so it is recomputed only after the all-FP64 solve and where tied DOFs were filled
     if (!o->mixed || c->dTieS) {
-        EF_CHECK(residual64(c, x, b, r64, s));
-        EF_CHECK(dot_host(c, r64, r64, &rr, s));
+        EF_CHECK(residual64(c, x, b, r64, &rr, s));
     }
     inf.iterations = total;
     inf.relResidual = sqrt(rr) / bnorm;

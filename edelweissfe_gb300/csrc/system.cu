@@ -126,12 +126,14 @@ ef_status ef_bsr_matvec(ef_ctx* c, const double* x, double* y, void* stream) {
 }
 
 // r = b - K x on free rows (0 on Dirichlet rows): with the exact FP64 tangent (matrix-free element
-// apply) when the system is stored in FP32, else with the stored system
-ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, cudaStream_t s) {
-    if (!c->exact)
-        return ef_launch_bsr_residual((int)c->nNodes, c->dRowPtr, c->dColIdx, c->dBsrVals, c->keFp64, x, b, c->dMask,
-                                      r, c->nSM, s);
-    double* y = c->w64[4];
+// apply) when the system is stored in FP32, else with the stored system; rr (host, may be null): r.r, then
+// with a synchronisation of the stream
+ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, double* rr, cudaStream_t s) {
+    if (!c->exact) {
+        EF_CHECK(ef_launch_bsr_residual((int)c->nNodes, c->dRowPtr, c->dColIdx, c->dBsrVals, c->keFp64, x, b, c->dMask, r,
+                                        c->nSM, s));
+        return rr ? dot_host(c, r, r, rr, s) : EF_OK;
+    }
     if (c->dTieS) {  // the element apply needs the tied DOFs filled from their masters
         EF_CUDA(cudaMemcpyAsync(c->dTieTmp, x, sizeof(double) * c->nDof, cudaMemcpyDeviceToDevice, s));
         EF_CHECK(ef_launch_tie_fill((int64_t)c->hTieS.size(), c->dTieS, c->dTieA, c->dTieB, c->dTieTmp, s));
@@ -144,14 +146,18 @@ ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, cud
         else
             EF_CHECK(ef_launch_small_strain_apply(g, x, c->dTang[gi], c->dYe + g.peOffset, s));
     }
-    EF_CHECK(ef_launch_condense(c->nNodes, c->dNodeDof, c->dCondPtr, c->dCondSrc, c->dCondW, c->dYe, y, nullptr, s));
-    return ef_launch_residual_from(c->nDof, b, y, c->dMask, r, s);
+    EF_CHECK(ef_launch_condense_residual(c->nNodes, c->dNodeDof, c->dCondPtr, c->dCondSrc, c->dCondW, c->dYe, b, c->dMask,
+                                         r, c->dPart, c->nPart, c->dTicket, rr ? c->hResDev->red : nullptr, s));
+    if (!rr) return EF_OK;
+    EF_CUDA(cudaStreamSynchronize(s));
+    *rr = c->hRes->red[0];
+    return EF_OK;
 }
 
 ef_status dot_host(ef_ctx* c, const double* a, const double* b, double* out, cudaStream_t s) {
-    EF_CHECK(ef_launch_dot(c->nDof, a, b, c->dPart, c->nPart, c->dRed, s));
-    EF_CUDA(cudaMemcpyAsync(out, c->dRed, sizeof(double), cudaMemcpyDeviceToHost, s));
+    EF_CHECK(ef_launch_dot(c->nDof, a, b, c->dPart, c->nPart, c->dTicket, c->hResDev->red, s));
     EF_CUDA(cudaStreamSynchronize(s));
+    *out = c->hRes->red[0];
     return EF_OK;
 }
 
@@ -177,27 +183,26 @@ ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIte
                          PcgResultHost* out, ef_solve_info* prof, cudaStream_t s) {
     void** w = vDouble ? c->w64k : c->w32;
     EF_CHECK(pcg_plan(c, vDouble));
+    c->hRes->pcg.status = -1;  // stays so when a CTA gave up waiting for the others
     if (prof) EF_CUDA(cudaEventRecord(c->ev[0], s));
     if (c->pcgSmem > 0)
         EF_CHECK(ef_launch_pcg_resident(vDouble, c->pcgShape, (int)c->nNodes, c->dRowPtr, c->dPcgLcol, c->dPcgHaloPtr,
                                         c->dPcgHaloIdx, c->dPcgGroupPtr, c->pcgSmem, c->dBsrVals, c->dBinv, c->dMask,
-                                        rhs, sol, w[3], c->dPcgSlots, c->dPcgRes, maxIter, rtol * rtol, c->dFlags, s));
+                                        rhs, sol, w[3], c->dPcgSlots, &c->hResDev->pcg, maxIter, rtol * rtol, c->dFlags, s));
     else
         EF_CHECK(ef_launch_pcg(vDouble, c->nSM, (int)c->nNodes, c->dRowPtr, c->dColIdx, c->dBsrVals, c->dBinv, c->dMask,
-                               rhs, sol, w[2], w[3], w[4], w[5], w[6], c->dPcgSlots, ef_pcg_slot_sets(), c->dPcgRes,
-                               maxIter, rtol * rtol, c->dFlags, s));
+                               rhs, sol, w[2], w[3], w[4], w[5], w[6], c->dPcgSlots, ef_pcg_slot_sets(),
+                               &c->hResDev->pcg, maxIter, rtol * rtol, c->dFlags, s));
     if (prof) EF_CUDA(cudaEventRecord(c->ev[1], s));
-    EF_CUDA(cudaMemcpyAsync(out, c->dPcgRes, sizeof(PcgResultHost), cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));
+    *out = c->hRes->pcg;
     if (prof) {
         float ms = 0.f;
         EF_CUDA(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
         prof->kernelMs += ms;
         prof->kernelLaunches += 1;
     }
-    int f = 0;
-    EF_CUDA(cudaMemcpy(&f, c->dFlags, sizeof(int), cudaMemcpyDeviceToHost));
-    if (f & EF_FLAG_BARRIER) {
+    if (out->status == -1) {
         ef_set_error("PCG: grid barrier timed out");
         return EF_ERR_DEVICE;
     }
@@ -221,19 +226,12 @@ ef_status ef_newton_residual(ef_ctx* c, int mode, const double* P, const double*
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (mode == 0) return ef_launch_newton_first(c->nDof, P, PExt, c->nDir, c->dDirIdx, dirValues, R, s);
-    if (!c->dNewton) {
-        ef_status st = EF_OK;
-        c->dNewton = dalloc<double>(16, &st);
-        if (!c->dNewton) return st;
-    }
-    const double q[9] = {o->fluxTol, o->fluxTolAlt, o->corrTol, o->fluxFloor, o->nAccFluxes, prevResidual,
-                         (double)iteration, (double)nGrew, ddU ? 1.0 : 0.0};
-    EF_CUDA(cudaMemcpyAsync(c->dNewton, q, sizeof(q), cudaMemcpyHostToDevice, s));
-    EF_CHECK(ef_launch_newton_check(c->nDof, P, PExt, c->dDirMask, F, ddU, R, c->dPart, c->nPart, c->dNewton,
-                                    c->dNewton + 9, s));
-    double r[5];
-    EF_CUDA(cudaMemcpyAsync(r, c->dNewton + 9, sizeof(r), cudaMemcpyDeviceToHost, s));
+    const NewtonTest q = {o->fluxTol, o->fluxTolAlt, o->corrTol, o->fluxFloor, o->nAccFluxes, prevResidual, iteration,
+                          nGrew};
+    EF_CHECK(ef_launch_newton_check(c->nDof, P, PExt, c->dDirMask, F, ddU, R, c->dPart, c->nPart, c->dTicket, q,
+                                    c->hResDev->red, s));
     EF_CUDA(cudaStreamSynchronize(s));
+    const double* r = c->hRes->red;
     out->converged = r[0] != 0.0;
     out->nGrew = (int)r[1];
     out->fluxResidual = r[2];
@@ -246,9 +244,9 @@ ef_status ef_norms(ef_ctx* c, const double* R, const double* F, const double* dd
     EF_REQUIRE_FINALIZED(c);
     if (!out) return EF_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    EF_CHECK(ef_launch_norms(c->nDof, R, F, ddU, c->dPart, c->nPart, c->dRed, s));
-    EF_CUDA(cudaMemcpyAsync(out, c->dRed, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    EF_CHECK(ef_launch_norms(c->nDof, R, F, ddU, c->dPart, c->nPart, c->dTicket, c->hResDev->red, s));
     EF_CUDA(cudaStreamSynchronize(s));
+    memcpy(out, c->hRes->red, 3 * sizeof(double));
     return EF_OK;
 }
 
