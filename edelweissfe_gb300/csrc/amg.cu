@@ -681,18 +681,17 @@ __device__ __forceinline__ float2 ldv2(const float* p) {
     return *reinterpret_cast<const float2*>(p);
 }
 // H: the block values come from a BF16 copy (valsH, 6 values = three 4-byte words per block row)
+// the sum over blocks first, first + step, ... (15 at a time) of a row
 template <bool CG, bool H = false>
-__device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __restrict__ rowPtr,
-                                           const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
-                                           const float* x, const float* r, const uint8_t* __restrict__ mask, float* t,
-                                           const float* __restrict__ binv, float omega,
-                                           const uint32_t* __restrict__ valsH = nullptr, float ys = 1.f) {
+__device__ __forceinline__ float resid6_sum(int m, int lane, int first, int step, const int32_t* __restrict__ rowPtr,
+                                            const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
+                                            const float* x, const uint32_t* __restrict__ valsH) {
     const int g = lane / BC, ri = lane - BC * g;
     float acc = 0.f;
     if (g < 5) {
         // three blocks per lane and step (15 per warp), their loads issued together
         const int e = rowPtr[m + 1];
-        for (int k0 = rowPtr[m] + g; k0 < e; k0 += 15) {
+        for (int k0 = rowPtr[m] + first + g; k0 < e; k0 += step) {
             int c[3];
             float2 a[3][3];
 #pragma unroll
@@ -728,7 +727,14 @@ __device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __res
     // lanes i < 6: acc(i) + acc(i + 6) + acc(i + 12) + acc(i + 18) + acc(i + 24)
     const float s1 = acc + __shfl_down_sync(0xffffffffu, acc, 6);
     const float s2 = s1 + __shfl_down_sync(0xffffffffu, s1, 12);
-    const float yi = s2 + __shfl_down_sync(0xffffffffu, acc, 24);
+    return s2 + __shfl_down_sync(0xffffffffu, acc, 24);
+}
+
+// the row's end: component i of the product, yi, in lane i < 6 of the warp
+template <bool CG>
+__device__ __forceinline__ void resid6_end(int m, int lane, float yi, const float* x, const float* r,
+                                           const uint8_t* __restrict__ mask, float* t, const float* __restrict__ binv,
+                                           float omega, float ys) {
     float y[BC];
 #pragma unroll
     for (int i = 0; i < BC; ++i) y[i] = __shfl_sync(0xffffffffu, yi, i);
@@ -740,6 +746,16 @@ __device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __res
             stv<CG>(t + d, (mask && mask[d]) ? 0.f : ldv<CG>(r + d) - ys * yi);
         }
     }
+}
+
+template <bool CG, bool H = false>
+__device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __restrict__ rowPtr,
+                                           const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
+                                           const float* x, const float* r, const uint8_t* __restrict__ mask, float* t,
+                                           const float* __restrict__ binv, float omega,
+                                           const uint32_t* __restrict__ valsH = nullptr, float ys = 1.f) {
+    const float yi = resid6_sum<CG, H>(m, lane, 0, 15, rowPtr, colIdx, vals, x, valsH);
+    resid6_end<CG>(m, lane, yi, x, r, mask, t, binv, omega, ys);
 }
 
 __global__ void __launch_bounds__(256) level_residual6_kernel(int nN, const int32_t* __restrict__ rowPtr,
@@ -757,6 +773,28 @@ __global__ void __launch_bounds__(256) level_residual6_kernel(int nN, const int3
         resid6_row<false, true>(m, lane, rowPtr, colIdx, vals, x, r, mask, t, binv, omega, valsH, ys);
     else
         resid6_row<false, false>(m, lane, rowPtr, colIdx, vals, x, r, mask, t, binv, omega, nullptr, ys);
+}
+
+// The same with W warps per row, for levels of too few rows to fill the GPU with a warp each (the row is then a
+// chain of dependent loads, 15 blocks at a time): warp w takes blocks 15 w, 15 (w + W), ... and warp 0
+// adds the warps' sums in order
+template <int W>
+__global__ void __launch_bounds__(32 * W) level_residual6_split_kernel(
+    int nN, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
+    const float* __restrict__ x, const float* __restrict__ r, const uint8_t* __restrict__ mask, float* __restrict__ t,
+    const float* __restrict__ binv, float omega, const uint32_t* __restrict__ valsH, float ys) {
+    ef::dep_entry();
+    __shared__ float part[W][BC];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = blockIdx.x;
+    float yi = valsH ? resid6_sum<false, true>(m, lane, 15 * w, 15 * W, rowPtr, colIdx, vals, x, valsH)
+                     : resid6_sum<false, false>(m, lane, 15 * w, 15 * W, rowPtr, colIdx, vals, x, nullptr);
+    if (lane < BC) part[w][lane] = yi;
+    __syncthreads();
+    if (w != 0) return;
+    if (lane < BC)
+#pragma unroll
+        for (int q = 1; q < W; ++q) yi += part[q][lane];
+    resid6_end<false>(m, lane, yi, x, r, mask, t, binv, omega, ys);
 }
 
 // B = A (M D^-1) on a 6-DOF level: block k of A times the block inverse of its column node with
@@ -806,21 +844,20 @@ __global__ void sa_post6_setup_kernel(int64_t nAP, const int32_t* __restrict__ a
 // a warp per row m; lanes 6 k + i (k < 5) take component i of the row's blocks k, k + 5, ...;
 // the five partial sums of a component are added in a fixed order, then lanes i < 6 form
 // x[m][i] = w (D_m^-1 (r + t)_m)[i] + y[i] (dead DOFs 0)
-__global__ void __launch_bounds__(256) sa_post6_fused_kernel(int nN, const int32_t* __restrict__ rowPtr,
-                                                             const int32_t* __restrict__ col,
-                                                             const float* __restrict__ C, const float* __restrict__ e,
-                                                             const float* __restrict__ r, const float* __restrict__ t,
-                                                             const float* __restrict__ binv,
-                                                             const uint8_t* __restrict__ dead, float omega,
-                                                             float* __restrict__ x) {
+// W warps per row (as level_residual6_split_kernel), or for W = 1 eight rows of a warp each per CTA
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W) sa_post6_fused_kernel(
+    int nN, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ col, const float* __restrict__ C,
+    const float* __restrict__ e, const float* __restrict__ r, const float* __restrict__ t,
+    const float* __restrict__ binv, const uint8_t* __restrict__ dead, float omega, float* __restrict__ x) {
     ef::dep_entry();
-    const int lane = threadIdx.x & 31;
-    const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31, w = W == 1 ? 0 : threadIdx.x >> 5;
+    const int m = W == 1 ? (blockIdx.x * blockDim.x + threadIdx.x) >> 5 : blockIdx.x;
     if (m >= nN) return;  // whole warps
     const int k0 = lane / BC, i = lane % BC;
     float y = 0.f;
     if (k0 < 5)
-        for (int a = rowPtr[m] + k0; a < rowPtr[m + 1]; a += 5) {
+        for (int a = rowPtr[m] + 5 * w + k0; a < rowPtr[m + 1]; a += 5 * W) {
             const float* cr = C + (int64_t)a * BC * BC + i * BC;
             const float* ev = e + BC * (int64_t)col[a];
 #pragma unroll
@@ -832,6 +869,15 @@ __global__ void __launch_bounds__(256) sa_post6_fused_kernel(int nN, const int32
     for (int k = 1; k < 5; ++k) {
         const float v = __shfl_sync(0xffffffffu, y, (i + BC * k) & 31);
         if (k0 == 0) s += v;
+    }
+    if (W > 1) {
+        __shared__ float part[W][BC];
+        if (lane < BC) part[w][lane] = s;
+        __syncthreads();
+        if (w != 0) return;
+        if (lane < BC)
+#pragma unroll
+            for (int q = 1; q < W; ++q) s += part[q][lane];
     }
     if (lane < BC) {
         const float* B = binv + (int64_t)m * BC * BC + i * BC;
@@ -1356,6 +1402,12 @@ static inline int nb_(int64_t n, int t) { return (int)((n + t - 1) / t); }
 int ef_amg_coarse_dofs() { return BC; }
 int ef_max_coarsest_nodes() { return kMaxCoarsestDof / BC; }
 
+// Warps per row of the 6-DOF levels' residual and post-smoothing: four for levels that a warp per row leaves with
+// less than about 13 warps an SM (preconditioner on the 300-node second level of 169,781 nodes 92.9 -> 91.6 us;
+// on the 6,664-node first level four warps cost 5.5 us)
+constexpr int kRowWarps = 4;
+static int row_warps(int nN) { return nN <= 2048 ? kRowWarps : 1; }
+
 ef_status ef_launch_galerkin(int bf, int64_t nCoarseBlocks, const int64_t* seg, const int32_t* src,
                              const int32_t* fineRowOfBlock, const int32_t* fineCol, const float* fineVals,
                              const uint8_t* fineMask, const float* offs, const int32_t* coarseRowOfBlock,
@@ -1401,8 +1453,12 @@ ef_status ef_launch_level_residual(int bs, int nN, const int32_t* rowPtr, const 
         EF_CUDA(ef::launch_dep(level_residual_kernel<3>, nb_((int64_t)nN * 8, 256), 256, 0, s, nN, rowPtr, colIdx, vals,
                 x, r, mask, t, binv, omega));
     } else {
-        EF_CUDA(ef::launch_dep(level_residual6_kernel, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, colIdx, vals,
-                x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
+        if (row_warps(nN) > 1)
+            EF_CUDA(ef::launch_dep(level_residual6_split_kernel<kRowWarps>, nN, 32 * kRowWarps, 0, s, nN, rowPtr, colIdx,
+                                   vals, x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
+        else
+            EF_CUDA(ef::launch_dep(level_residual6_kernel, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, colIdx, vals,
+                                   x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
     }
     EF_CUDA(cudaGetLastError());
     return EF_OK;
@@ -1430,8 +1486,12 @@ ef_status ef_launch_sa_post6_fused(int nN, const int32_t* rowPtr, const int32_t*
                                    const float* r, const float* t, const float* binv, const uint8_t* dead,
                                    float omega, float* x, cudaStream_t s) {
     if (nN <= 0) return EF_OK;
-    EF_CUDA(ef::launch_dep(sa_post6_fused_kernel, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, col, C, e, r, t,
-                           binv, dead, omega, x));
+    if (row_warps(nN) > 1)
+        EF_CUDA(ef::launch_dep(sa_post6_fused_kernel<kRowWarps>, nN, 32 * kRowWarps, 0, s, nN, rowPtr, col, C, e, r, t,
+                               binv, dead, omega, x));
+    else
+        EF_CUDA(ef::launch_dep(sa_post6_fused_kernel<1>, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, col, C, e, r,
+                               t, binv, dead, omega, x));
     return EF_OK;
 }
 
@@ -1553,8 +1613,11 @@ ef_status ef_launch_sa_restrict_onepass_h(int nC, const int32_t* tPtr, const int
                                           const void* q1, const void* q2, const float* t, const uint8_t* coarseDead,
                                           float* rc, cudaStream_t s) {
     if (nC <= 0) return EF_OK;
-    const char* e = getenv("EF_SA_RESTRICT_WARP");  // read at each launch site (the cycle is captured once)
-    const bool warp = !e || atoi(e) != 0;
+    // a warp per coarse node, or below about 16 of them an SM a CTA per coarse node (preconditioner at 3,400 coarse
+    // nodes 59.7 against 60.6 us, at 1,500 44.8 against 40.8, at 690 42.2 against 37.8); EF_SA_RESTRICT_WARP=1 / 0
+    // forces one (read at each launch site: the cycle is captured once)
+    const char* e = getenv("EF_SA_RESTRICT_WARP");
+    const bool warp = e ? atoi(e) != 0 : nC > 2400;
     if (warp)
         EF_CUDA(ef::launch_dep(sa_restrict_warp_h_kernel, nb_(nC, kSaRestrictWarpNodes), 32 * kSaRestrictWarpNodes,
                                0, s, nC, tPtr, rowT, (const uint4*)q0, (const uint4*)q1, (const uint32_t*)q2, t,

@@ -72,11 +72,18 @@ static ef_status sell_build(ef_ctx* c) {
     auto split = [](const char* e, int dflt) {
         if (!e) return dflt;
         const int k = atoi(e);
-        return (k == 1 || k == 2 || k == 4 || k == 8) ? k : dflt;
+        return (k == 1 || k == 2 || k == 4 || k == 8 || k == 16 || k == 32) ? k : dflt;
     };
-    c->sellSplit = split(getenv("EF_SELL_SPLIT"), c->sellSplit);
-    c->sellSplitProduct = split(getenv("EF_SELL_SPLIT_PRODUCT"), c->sellSplitProduct);
     const int n0 = (int)c->nNodes;
+    // Warps per slice: as many as it takes to give an SM enough warps to hide a step's loads, and no more (they
+    // meet in shared memory).  us of the product / the preconditioner with 4, 8 and 16 warps: 4,225 nodes 8.4 / 24.1,
+    // 8.0 / 21.4, 7.3 / 21.2; 18,081 nodes 12.6 / 37.8, 10.4 / 33.5, 9.7 / 31.2; 88,209 nodes 24.7 / 60.6,
+    // 23.0 / 59.8, 25.0 / 63.0; 169,781 nodes 35.4 / 83.6, 36.1 / 88.0, 41.3 / 101; rows of quadratic elements (up to
+    // 81 blocks) 7,500 nodes 28.5, 17.9 and 12.7 (32 warps: 10.4) for the product
+    const int perSM = (n0 + 32 * c->nSM - 1) / (32 * c->nSM);  // slices
+    const int warps = perSM <= 6 ? 16 : (perSM <= 24 ? 8 : 4);
+    c->sellSplit = split(getenv("EF_SELL_SPLIT"), warps);
+    c->sellSplitProduct = split(getenv("EF_SELL_SPLIT_PRODUCT"), perSM <= 2 ? 32 : warps);
     const std::vector<int32_t>& rp = c->hRowPtr0;
     const std::vector<int32_t>& ci = c->hColIdx0;
     if (c->keFp64 || n0 <= 0 || (int64_t)rp.size() != (int64_t)n0 + 1) return EF_OK;

@@ -382,6 +382,10 @@ ef_status ef_launch_sell_spmv3(int nN, int nSlices, const int64_t* off, const in
         EF_SPMV3(C_, 4);    \
     else if (split == 8)    \
         EF_SPMV3(C_, 8);    \
+    else if (split == 16)   \
+        EF_SPMV3(C_, 16);   \
+    else if (split == 32)   \
+        EF_SPMV3(C_, 32);   \
     else                    \
         EF_SPMV3(C_, 1)
     if (xcopy) {
@@ -417,6 +421,10 @@ ef_status ef_launch_sell_level3_bf16(int nN, int nSlices, const int64_t* off, co
         EF_L3(2);
     else if (split == 8)
         EF_L3(8);
+    else if (split == 16)
+        EF_L3(16);
+    else if (split == 32)
+        EF_L3(32);
     else
         EF_L3(4);
 #undef EF_L3
@@ -449,6 +457,8 @@ ef_status ef_launch_sa_post_fused(int nN, int nSlices, const int64_t* off, const
         EF_POST(2);
     else if (split == 8)
         EF_POST(8);
+    else if (split >= 16)
+        EF_POST(16);
     else
         EF_POST(4);
 #undef EF_POST
