@@ -36,3 +36,25 @@ def test_fgmres_with_every_split_solves_the_fp64_system(gpu_lib, monkeypatch, el
     _lib.check(f.lib.ef_bsr_matvec(f.ctx, x.data_ptr(), y.data_ptr(), f._stream()), "ef_bsr_matvec")
     assert float((b - y).norm() / b.norm()) <= 1e-7
     assert s.lastSolveInfo.relResidual <= 1e-8
+
+
+@pytest.mark.parametrize("dims", [(2, 1, 1), (50, 16, 16), (60, 20, 20)], ids=lambda d: "x".join(map(str, d)))
+def test_fgmres_gram_schmidt_of_every_vector_length(gpu_lib, dims):
+    """Vectors of 36, 44,217 and 80,703 elements: the basis dealt out over four, two and one set of threads
+    (13,000 elements above: four); more columns than are loaded ahead.  The same check."""
+    from edelweissfe_gb300 import _lib
+    from edelweissfe_gb300.solver import LinSolverOptions, TimeStep
+
+    spec = j2_box_spec(*dims, *[0.1 * k for k in dims])
+    ts = TimeStep(1, 0.1, 0.1, 0.1, 0.1, 0.1)
+    s = build_gpu_solver(spec, linsolver=LinSolverOptions(method="fgmres", rtol=1e-8, innerRtol=1e-7, restart=100))
+    f = build_gpu_solver(spec, keFp64=True, linsolver=LinSolverOptions(mixed=False))
+    b = torch.as_tensor(np.random.default_rng(9).normal(size=s.nDof), device="cuda")
+    b[s.dirIdx] = 0.0
+    for g in (s, f):
+        d, P, F = g._vec(), g._vec(), g._vec()
+        g.computeElements(d, d, P, F, ts)
+        g.assembleStiffnessCSR()
+    x, y = s.linearSolve(b), s._vec()
+    _lib.check(f.lib.ef_bsr_matvec(f.ctx, x.data_ptr(), y.data_ptr(), f._stream()), "ef_bsr_matvec")
+    assert float((b - y).norm() / b.norm()) <= 1e-7
