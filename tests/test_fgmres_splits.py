@@ -38,9 +38,9 @@ def test_fgmres_with_every_split_solves_the_fp64_system(gpu_lib, monkeypatch, el
     assert s.lastSolveInfo.relResidual <= 1e-8
 
 
-@pytest.mark.parametrize("dims", [(2, 1, 1), (50, 16, 16), (60, 20, 20)], ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("dims", [(4, 2, 2), (50, 16, 16), (60, 20, 20)], ids=lambda d: "x".join(map(str, d)))
 def test_fgmres_gram_schmidt_of_every_vector_length(gpu_lib, dims):
-    """Vectors of 36, 44,217 and 80,703 elements: the basis dealt out over four, two and one set of threads
+    """Vectors of 135, 44,217 and 80,703 elements: the basis dealt out over four, two and one set of threads
     (13,000 elements above: four); more columns than are loaded ahead.  The same check."""
     from edelweissfe_gb300 import _lib
     from edelweissfe_gb300.solver import LinSolverOptions, TimeStep
