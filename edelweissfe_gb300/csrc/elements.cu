@@ -169,38 +169,41 @@ __global__ void geometry_kernel(const ElemTables* __restrict__ T, int nEl, const
     }
 }
 
-// a split value in the stiffness precision: hi for FP32, hi + lo for FP64
-template <typename KT>
-__device__ __forceinline__ KT gk_value(float2 v);
-template <>
-__device__ __forceinline__ float gk_value<float>(float2 v) {
-    return v.x;
-}
-template <>
-__device__ __forceinline__ double gk_value<double>(float2 v) {
-    return (double)v.x + (double)v.y;
+// x with its sign flipped where neg has the sign bit (integer pipe)
+__device__ __forceinline__ double flip_sign(double x, int neg) {
+    return __hiloint2double(__double2hiint(x) ^ neg, __double2loint(x));
 }
 
 template <int NN, int NQ, typename KT>
 struct SSShared {
     static constexpr int TPE = (NQ <= 8) ? 8 : 32;
-    static constexpr int EPB = kBlock / TPE;
+    // two elements a CTA for the FP64 stiffness of up to 27 Gauss points, whose scratch is twice as large
+    static constexpr int BLOCK = (TPE == 32 && sizeof(KT) == 8) ? 64 : kBlock;
+    static constexpr int EPB = BLOCK / TPE;
+    static constexpr int NG = NQ * NN * 3 + 1;
     // per-element rows padded by one entry, so that the elements of a warp fall on different banks
     float2 du[EPB][NN * 3 + 1];       // dU split into FP32 pairs, [3a + i]
-    float2 g[EPB][NQ * NN * 3 + 1];   // dN/dx split into FP32 pairs, [(q NN + a) 3 + c] (the FP32 stiffness reads hi)
     float2 sw[EPB][NQ * 6 + 1];       // sigma w detJ split into FP32 pairs, [6q + i]
-    KT tn[EPB][NQ][9];                // lt*w, mt*w, c1*w, n[6]
+    KT tn[EPB][NQ][9];                // FP32: lt*w, mt*w, c1*w, n[6]; FP64: c2, c1, w (its sign)
+    union {
+        float2 g[EPB][NG];            // dN/dx split into FP32 pairs, [(q NN + a) 3 + c] (the FP32 stiffness reads hi)
+        struct {                      // the FP64 stiffness, once the residual is done with g
+            double gd[EPB][NG];       // sqrt(|w detJ|) dN/dx
+            double vd[sizeof(KT) == 8 ? EPB : 1][sizeof(KT) == 8 ? NG : 1];  // n . gd, where plastic
+        } d;
+    } u;
 };
 
 // Element loop of one group: strain increment, constitutive update, Pe (FP64) and Ke blocks (KT).
 template <int NN, int NQ, typename KT, int MAT, bool VIJ>
-__global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
-    int nEl, const int32_t* __restrict__ nodeDof, const float2* __restrict__ geoS, const double* __restrict__ dU,
+__global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ? (NQ <= 8 ? 3 : 4) : 5) small_strain_kernel(
+    int nEl, const int32_t* __restrict__ nodeDof, const float2* __restrict__ geoS, const double* __restrict__ geo,
+    const double* __restrict__ dU,
     const double* __restrict__ stateIn, double* __restrict__ stateOut, PropsArg props,
     const double* __restrict__ propsTable, const int32_t* __restrict__ elemRow, KT* __restrict__ Kout,
     double* __restrict__ Pe, double* __restrict__ tang, int* __restrict__ flags, int intConv) {
     constexpr int TPE = (NQ <= 8) ? 8 : 32;
-    constexpr int EPB = kBlock / TPE;
+    constexpr int EPB = SSShared<NN, NQ, KT>::EPB;
     constexpr int NP = PairTab<NN>::NP;
     constexpr int ND = 3 * NN;
     constexpr int NG = 3 * NN + 1;
@@ -222,6 +225,9 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
     }
     __syncthreads();
 
+    MatOut mo;
+    mo.c1 = mo.c2 = 0.0;
+    const double* pv = propsTable ? propsTable + 8 * (int64_t)elemRow[valid ? e : 0] : props.v;
     // ---- Gauss-point phase ---------------------------------------------------
     if (valid && lane < NQ) {
         const int q = lane;
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 ga[c] = gq[3 * a + c];
-                sh.g[le][(q * NN + a) * 3 + c] = ga[c];
+                sh.u.g[le][(q * NN + a) * 3 + c] = ga[c];
             }
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -259,8 +265,6 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
         double sig[6];
 #pragma unroll
         for (int i = 0; i < 6; ++i) sig[i] = stateIn[i * nQPtot + qi];
-        MatOut mo;
-        const double* pv = propsTable ? propsTable + 8 * (int64_t)elemRow[e] : props.v;
         if (MAT == MAT_VON_MISES) {
             double kap = stateIn[12 * nQPtot + qi];
             if (!mat_von_mises(pv, sig, &kap, de, mo)) {
@@ -288,24 +292,29 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
 #pragma unroll
             for (int i = 0; i < 6; ++i) tang[(3 + i) * nQPtot + qi] = mo.c1 != 0.0 ? mo.n[i] : 0.0;
         }
-        sh.tn[le][q][0] = (KT)(mo.lt * wdet);
-        sh.tn[le][q][1] = (KT)(mo.mt * wdet);
-        sh.tn[le][q][2] = (KT)(mo.c1 * wdet);
-        if (mo.c1 != 0.0) {
+        if (sizeof(KT) == 8) {
+            sh.tn[le][q][0] = (KT)mo.c2;
+            sh.tn[le][q][1] = (KT)mo.c1;
+            sh.tn[le][q][2] = (KT)wdet;
+        } else {
+            sh.tn[le][q][0] = (KT)(mo.lt * wdet);
+            sh.tn[le][q][1] = (KT)(mo.mt * wdet);
+            sh.tn[le][q][2] = (KT)(mo.c1 * wdet);
+            if (mo.c1 != 0.0) {
 #pragma unroll
-            for (int i = 0; i < 6; ++i) sh.tn[le][q][3 + i] = (KT)mo.n[i];
+                for (int i = 0; i < 6; ++i) sh.tn[le][q][3 + i] = (KT)mo.n[i];
+            }
         }
     }
     __syncthreads();
-    if (!valid) return;
 
     // ---- residual: Pe_a = -sum_q (sigma w detJ) . g_qa  (double-float accumulation) ----
-    for (int a = lane; a < NN; a += TPE) {
+    for (int a = valid ? lane : NN; a < NN; a += TPE) {
         DF f0{0.f, 0.f}, f1{0.f, 0.f}, f2{0.f, 0.f};
 #pragma unroll 2
         for (int q = 0; q < NQ; ++q) {
             const float2* s = &sh.sw[le][6 * q];
-            const float2* gg = &sh.g[le][(q * NN + a) * 3];
+            const float2* gg = &sh.u.g[le][(q * NN + a) * 3];
             const float2 gx = gg[0], gy = gg[1], gz = gg[2];
             df_fma(f0, s[0], gx);
             df_fma(f0, s[3], gy);
@@ -323,6 +332,113 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
         pe[2] = -df_value_sel(f2, intConv);
     }
 
+    auto store = [&](int p, int a, int b, const KT (&k)[3][3]) {
+        if (VIJ) {
+            // reference VIJ layout: value a*n+b of the element slice holds Ke[a][b]
+            KT* ke = Kout + (int64_t)e * ND * ND;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    ke[(3 * a + i) * ND + 3 * b + j] = k[i][j];
+                    if (a != b) ke[(3 * b + j) * ND + 3 * a + i] = k[i][j];
+                }
+        } else {
+            KT* kb = Kout + ((int64_t)e * NP + p) * 9;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) kb[i * 3 + j] = k[i][j];
+        }
+    };
+    if constexpr (sizeof(KT) == 8) {
+        // ---- stiffness in FP64, which the FP64 pipe bounds: K_ab = sum_q lt ga(x)gb + mt (gb(x)ga + ga.gb I)
+        // - c1 va(x)vb with lt = lam + c2/3, mt = G - c2/2 and lam, G of the element, so that
+        //   K = lam A + G (A^T + tr A I) + B/3 - (B^T + tr B I)/2 - V,
+        //   A = sum_q ga(x)gb, B = sum_q c2 ga(x)gb, V = sum_q c1 va(x)vb, g with sqrt(|w detJ|) in it and the sign
+        // of w detJ (negative in an inverted element, which the element status reports) given to ga and va:
+        // 9 instructions per pair of nodes and elastic Gauss point, 33 where plastic, against 58 and 88 with the
+        // three terms formed per pair from the split geometry (10,240 hex8 J2 elements, half of them plastic: 659 ->
+        // 326 us with the FP64 pipe 87 % busy before).  The FP64 geometry (not its 48-bit split) is
+        // scaled once per Gauss point and node, va = n . ga likewise.
+        __syncthreads();  // the residual has read g
+        if (valid && lane < NQ) {
+            const int q = lane;
+            const double* gq = geo + ((int64_t)e * NQ + q) * (3 * NN + 1);
+            const double sw = sqrt(fabs(gq[3 * NN]));
+#pragma unroll 2
+            for (int a = 0; a < NN; ++a) {
+                const double g0 = sw * gq[3 * a], g1 = sw * gq[3 * a + 1], g2 = sw * gq[3 * a + 2];
+                double* gd = &sh.u.d.gd[le][(q * NN + a) * 3];
+                gd[0] = g0;
+                gd[1] = g1;
+                gd[2] = g2;
+                if (mo.c1 != 0.0 || mo.c2 != 0.0) {
+                    double* vd = &sh.u.d.vd[le][(q * NN + a) * 3];
+                    vd[0] = fma(mo.n[4], g2, fma(mo.n[3], g1, mo.n[0] * g0));
+                    vd[1] = fma(mo.n[5], g2, fma(mo.n[1], g1, mo.n[3] * g0));
+                    vd[2] = fma(mo.n[2], g2, fma(mo.n[5], g1, mo.n[4] * g0));
+                }
+            }
+        }
+        __syncthreads();
+        if (!valid) return;
+        const double lam = pv[6], G = pv[7];
+        for (int p = lane; p < NP; p += TPE) {
+            const int a = pair_a(p, NN);
+            const int b = a + (p - (a * NN - a * (a - 1) / 2));
+            double A[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, B[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+            double V[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+            bool plastic = false;
+            for (int q = 0; q < NQ; ++q) {
+                const double* gA = &sh.u.d.gd[le][(q * NN + a) * 3];
+                const double* gB = &sh.u.d.gd[le][(q * NN + b) * 3];
+                const int neg = __double2hiint(sh.tn[le][q][2]) & 0x80000000;
+                const double ga[3] = {flip_sign(gA[0], neg), flip_sign(gA[1], neg), flip_sign(gA[2], neg)};
+                const double gb[3] = {gB[0], gB[1], gB[2]};
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) A[i][j] = fma(ga[i], gb[j], A[i][j]);
+                const double c2 = sh.tn[le][q][0], c1 = sh.tn[le][q][1];
+                if (MAT == MAT_VON_MISES && (__double2hiint(c2) | __double2hiint(c1)) != 0) {
+                    plastic = true;
+                    const double* vA = &sh.u.d.vd[le][(q * NN + a) * 3];
+                    const double* vB = &sh.u.d.vd[le][(q * NN + b) * 3];
+                    const double cg[3] = {c2 * ga[0], c2 * ga[1], c2 * ga[2]};
+                    const double c1s = flip_sign(c1, neg);
+                    const double cv[3] = {c1s * vA[0], c1s * vA[1], c1s * vA[2]};
+                    const double vb[3] = {vB[0], vB[1], vB[2]};
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            B[i][j] = fma(cg[i], gb[j], B[i][j]);
+                            V[i][j] = fma(cv[i], vb[j], V[i][j]);
+                        }
+                }
+            }
+            KT k[3][3];
+            const double s = G * (A[0][0] + A[1][1] + A[2][2]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) k[i][j] = fma(G, A[j][i], i == j ? fma(lam, A[i][j], s) : lam * A[i][j]);
+            if (plastic) {
+                const double h = -0.5 * (B[0][0] + B[1][1] + B[2][2]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const double t = fma(-0.5, B[j][i], fma(1.0 / 3.0, B[i][j], (i == j ? h : 0.0) - V[i][j]));
+                        k[i][j] += t;
+                    }
+            }
+            store(p, a, b, k);
+        }
+        return;
+    }
+    if (!valid) return;
     // ---- stiffness: K_ab = sum_q lt ga(x)gb + mt (gb(x)ga + ga.gb I) - c1 va(x)vb ----
     for (int p = lane; p < NP; p += TPE) {
         const int a = pair_a(p, NN);
@@ -330,10 +446,10 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
         KT k[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
         for (int q = 0; q < NQ; ++q) {
             const KT* tn = sh.tn[le][q];
-            const float2* gA = &sh.g[le][(q * NN + a) * 3];
-            const float2* gB = &sh.g[le][(q * NN + b) * 3];
-            const KT ga0 = gk_value<KT>(gA[0]), ga1 = gk_value<KT>(gA[1]), ga2 = gk_value<KT>(gA[2]);
-            const KT gb0 = gk_value<KT>(gB[0]), gb1 = gk_value<KT>(gB[1]), gb2 = gk_value<KT>(gB[2]);
+            const float2* gA = &sh.u.g[le][(q * NN + a) * 3];
+            const float2* gB = &sh.u.g[le][(q * NN + b) * 3];
+            const KT ga0 = (KT)gA[0].x, ga1 = (KT)gA[1].x, ga2 = (KT)gA[2].x;
+            const KT gb0 = (KT)gB[0].x, gb1 = (KT)gB[1].x, gb2 = (KT)gB[2].x;
             const KT lt = tn[0], mt = tn[1], c1 = tn[2];
             const KT s = mt * (ga0 * gb0 + ga1 * gb1 + ga2 * gb2);
             const KT la[3] = {lt * ga0, lt * ga1, lt * ga2};
@@ -358,23 +474,7 @@ __global__ void __launch_bounds__(kBlock, 5) small_strain_kernel(
                     for (int j = 0; j < 3; ++j) k[i][j] -= c1 * va[i] * vb[j];
             }
         }
-        if (VIJ) {
-            // reference VIJ layout: value a*n+b of the element slice holds Ke[a][b]
-            KT* ke = Kout + (int64_t)e * ND * ND;
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    ke[(3 * a + i) * ND + 3 * b + j] = k[i][j];
-                    if (a != b) ke[(3 * b + j) * ND + 3 * a + i] = k[i][j];
-                }
-        } else {
-            KT* kb = Kout + ((int64_t)e * NP + p) * 9;
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) kb[i * 3 + j] = k[i][j];
-        }
+        store(p, a, b, k);
     }
 }
 
@@ -742,13 +842,15 @@ static ef_status launch_ss(const Group& g, const double* dU, void* K, int vij, d
     if (vij) {
         auto k = small_strain_kernel<NN, NQ, KT, MAT, true>;
         EF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kBlock, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geoS, dU, sIn, sOut, pa, g.propsTable, g.elemRow,
-                                                  (KT*)K, Pe, tang, flags, g.intConv);
+        k<<<grid, SSShared<NN, NQ, KT>::BLOCK, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geoS, g.geo, dU, sIn, sOut, pa,
+                                                                       g.propsTable, g.elemRow, (KT*)K, Pe, tang, flags,
+                                                                       g.intConv);
     } else {
         auto k = small_strain_kernel<NN, NQ, KT, MAT, false>;
         EF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kBlock, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geoS, dU, sIn, sOut, pa, g.propsTable, g.elemRow,
-                                                  (KT*)K, Pe, tang, flags, g.intConv);
+        k<<<grid, SSShared<NN, NQ, KT>::BLOCK, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geoS, g.geo, dU, sIn, sOut, pa,
+                                                                       g.propsTable, g.elemRow, (KT*)K, Pe, tang, flags,
+                                                                       g.intConv);
     }
     EF_CUDA(cudaGetLastError());
     return EF_OK;

@@ -24,6 +24,7 @@ namespace ef {
 
 struct MatOut {
     double lt, mt, c1;  // tangent C = lt 1x1 + 2 mt I_s - c1 n x n (Voigt, engineering shear)
+    double c2;          // lt = lambda + c2 / 3, mt = G - c2 / 2 (0 where elastic)
     double n[6];
 };
 
@@ -42,6 +43,7 @@ EF_MAT_HD void mat_linear_elastic(const double* props, double* sig, const double
     o.lt = lam;
     o.mt = mu;
     o.c1 = 0.0;
+    o.c2 = 0.0;
 }
 
 // J2 radial return with isotropic hardening fy = fy0 + H k + dfy (1 - exp(-delta k)) (vonmises.py:186-254)
@@ -52,6 +54,7 @@ EF_MAT_HD bool mat_von_mises(const double* props, double* sig, double* kappa, co
     o.lt = lam;
     o.mt = G;
     o.c1 = 0.0;
+    o.c2 = 0.0;
     const double nde2 = de[0] * de[0] + de[1] * de[1] + de[2] * de[2] + de[3] * de[3] + de[4] * de[4] + de[5] * de[5];
     if (nde2 < 1e-28) return true;  // zero-increment shortcut |de| < 1e-14: stress and kappa unchanged, C = Ei
     double t[6];
@@ -99,6 +102,7 @@ EF_MAT_UNROLL
         const double c1 = 2.0 * G * (1.0 / (1.0 + hp / (3.0 * G)) - 2.0 * G * dLam * inv);
         const double c2 = 4.0 * G * G * dLam * inv;
         o.c1 = c1;
+        o.c2 = c2;
         o.lt = lam + c2 * (1.0 / 3.0);
         o.mt = G - 0.5 * c2;
     } else {
