@@ -268,7 +268,9 @@ void ef_destroy(ef_ctx* c) {
     F(c->dIndices);
     F(c->dCsrSeg);
     F(c->dCsrPerm);
-    F(c->dKvijTmp);
+    F(c->dCsrRows);
+    if (c->hCsrRows) cudaFreeHost(c->hCsrRows);
+    if (c->csrRowsDone) cudaEventDestroy(c->csrRowsDone);
     F(c->dPart);
     F(c->dTicket);
     if (c->hRes) cudaFreeHost(c->hRes);

@@ -424,7 +424,9 @@ struct ef_ctx {
     int32_t* dIndices = nullptr;
     int64_t* dCsrSeg = nullptr;
     int32_t* dCsrPerm = nullptr;
-    double* dKvijTmp = nullptr;
+    int64_t *dCsrRows = nullptr, *hCsrRows = nullptr;  // rows of the last ef_csr_dirichlet_rows
+    int64_t csrRowsCap = 0;
+    cudaEvent_t csrRowsDone = nullptr;  // their last launch
     // reductions / Krylov workspace
     double* dPart = nullptr;
     int nPart = 0;

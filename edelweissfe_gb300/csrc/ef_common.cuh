@@ -115,6 +115,13 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 #endif
 
+// The element groups as the scalar CSR scatter sees them: where a group's VIJ values end and its blocks begin
+struct CsrGroups {
+    int n;
+    int vijEnd[EF_MAX_GROUPS], nd[EF_MAX_GROUPS];
+    int64_t keOffset[EF_MAX_GROUPS];
+};
+
 // Inputs of the Newton check (ef_newton_residual)
 struct NewtonTest {
     double fluxTol, fluxTolAlt, corrTol, fluxFloor, nAccFluxes, prevResidual;
@@ -180,6 +187,8 @@ ef_status ef_launch_results_gather(int64_t nPts, int nQ, int nQP, int64_t nq, in
                                    cudaStream_t s);
 ef_status ef_launch_csr_scatter(int64_t nnz, const int64_t* seg, const int32_t* perm, const double* V, double* data,
                                 cudaStream_t s);
+ef_status ef_launch_csr_from_blocks(int64_t nnz, const int64_t* seg, const int32_t* perm, const ef::CsrGroups& G,
+                                    const void* Kblk, int kDouble, double* data, cudaStream_t s);
 ef_status ef_launch_csr_dirichlet_rows(int64_t nRows, const int64_t* rows, const int32_t* indptr,
                                        const int32_t* indices, double* data, cudaStream_t s);
 ef_status ef_launch_tie_fill(int64_t n, const int32_t* slave, const int32_t* ma, const int32_t* mb, double* x,

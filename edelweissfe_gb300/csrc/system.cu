@@ -35,14 +35,14 @@ ef_status ef_update_csr(ef_ctx* c, const double* Kvij, double* csrData, void* st
         return EF_ERR_STATE;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (!Kvij) {
-        if (!c->dKvijTmp) {
-            ef_status st = EF_OK;
-            c->dKvijTmp = dalloc<double>(c->nVIJ, &st);
-            if (!c->dKvijTmp) return st;
+    if (!Kvij) {  // the context's own element blocks, without the VIJ vector between
+        CsrGroups G = {};
+        for (const auto& g : c->groups) {
+            G.vijEnd[G.n] = (int)((G.n ? G.vijEnd[G.n - 1] : 0) + (int64_t)g.nEl * g.nDofEl * g.nDofEl);
+            G.nd[G.n] = g.nDofEl;
+            G.keOffset[G.n++] = g.keOffset;
         }
-        EF_CHECK(ef_export_vij(c, c->dKvijTmp, stream));
-        Kvij = c->dKvijTmp;
+        return ef_launch_csr_from_blocks(c->nnz, c->dCsrSeg, c->dCsrPerm, G, c->Kblk, c->keFp64, csrData, s);
     }
     return ef_launch_csr_scatter(c->nnz, c->dCsrSeg, c->dCsrPerm, Kvij, csrData, s);
 }
@@ -56,15 +56,27 @@ ef_status ef_csr_dirichlet_rows(ef_ctx* c, double* csrData, const int64_t* rows,
             ef_set_error("ef_csr_dirichlet_rows: row out of range");
             return EF_ERR_ARG;
         }
-    ef_status st = EF_OK;
-    int64_t* d = dalloc<int64_t>(nRows, &st);
-    if (!d) return st;
+    // the rows go through buffers of the context (no allocation and no synchronisation per call): a pinned copy, so
+    // that the caller's array is free again, and a device one; both wait for the launch that last used them
     cudaStream_t s = (cudaStream_t)stream;
-    cudaMemcpyAsync(d, rows, sizeof(int64_t) * nRows, cudaMemcpyHostToDevice, s);
-    st = ef_launch_csr_dirichlet_rows(nRows, d, c->dIndptr, c->dIndices, csrData, s);
-    cudaStreamSynchronize(s);
-    cudaFree(d);
-    return st;
+    if (!c->csrRowsDone) EF_CUDA(cudaEventCreateWithFlags(&c->csrRowsDone, cudaEventDisableTiming));
+    EF_CUDA(cudaEventSynchronize(c->csrRowsDone));
+    if (c->csrRowsCap < nRows) {
+        if (c->dCsrRows) cudaFree(c->dCsrRows);
+        if (c->hCsrRows) cudaFreeHost(c->hCsrRows);
+        c->dCsrRows = c->hCsrRows = nullptr;
+        c->csrRowsCap = 0;
+        ef_status st = EF_OK;
+        c->dCsrRows = dalloc<int64_t>(nRows, &st);
+        if (!c->dCsrRows) return st;
+        EF_CUDA(cudaHostAlloc((void**)&c->hCsrRows, sizeof(int64_t) * nRows, cudaHostAllocDefault));
+        c->csrRowsCap = nRows;
+    }
+    memcpy(c->hCsrRows, rows, sizeof(int64_t) * nRows);
+    EF_CUDA(cudaMemcpyAsync(c->dCsrRows, c->hCsrRows, sizeof(int64_t) * nRows, cudaMemcpyHostToDevice, s));
+    EF_CHECK(ef_launch_csr_dirichlet_rows(nRows, c->dCsrRows, c->dIndptr, c->dIndices, csrData, s));
+    EF_CUDA(cudaEventRecord(c->csrRowsDone, s));
+    return EF_OK;
 }
 
 ef_status ef_set_dirichlet(ef_ctx* c, const int64_t* dofs, int64_t n) {
