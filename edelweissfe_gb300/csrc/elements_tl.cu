@@ -20,11 +20,12 @@
 
 #include <math.h>
 
+#include "dfloat_bits.h"
 #include "ef_common.cuh"
 
 namespace ef {
 
-constexpr int kTLBlock = 128;
+constexpr int kTLBlock = 64;  // two elements of 27 Gauss points, eight of 8: the scratch of more leaves an SM one CTA
 
 __device__ __forceinline__ int tl_pair_a(int p, int nn) {
     int a = 0;
@@ -36,16 +37,49 @@ __device__ __forceinline__ int tl_pair_a(int p, int nn) {
     return a;
 }
 
+// Geometry of the stiffness in its own precision: the material gradients g0 (FP32: split into pairs hi, lo, for
+// the dot products g0_a . g0_b in double-float arithmetic) and the spatial gradients g of a node as the
+// first factor of a pair, and mb w detJ g and lb w detJ g as the second
+template <typename KT, int EPB, int NG>
+struct TLStiff;
+template <int EPB, int NG>
+struct TLStiff<double, EPB, NG> {
+    double g0[EPB][NG], gm[EPB][NG], gl[EPB][NG];
+};
+template <int EPB, int NG>
+struct TLStiff<float, EPB, NG> {
+    float2 g0[EPB][NG];
+    float ga[EPB][NG], gm[EPB][NG], gl[EPB][NG];
+};
+
 template <int NN, int NQ, typename KT>
 struct TLShared {
-    static constexpr int TPE = (NQ <= 8) ? 8 : 32;
-    static constexpr int EPB = kTLBlock / TPE;
+    // threads per element: enough for its Gauss points and few idle in the last round of its pairs where the FP64 pipe
+    // counts; four warps for the FP32 stiffness of up to 27 Gauss points, whose scratch leaves an SM few elements
+    // (3,375 hex20 elements 342 us with one warp, 301 with four)
+    static constexpr int TPE = (NQ <= 8) ? 8 : (sizeof(KT) == 8 ? 32 : 128);
+    static constexpr int BLOCK = TPE > kTLBlock ? TPE : kTLBlock;
+    static constexpr int EPB = BLOCK / TPE;
+    static constexpr int NG = NQ * NN * 3 + 1;
     double u[EPB][NN][3];
-    double g0[EPB][NQ][NN][3];
-    double g[EPB][NQ][NN][3];
-    double tw[EPB][NQ][6];  // tau * w detJ (11,22,33,12,23,13)
-    KT sc[EPB][NQ][3];      // mu w detJ, mb w detJ, lb w detJ
+    double g[EPB][NG];       // F^-T g0, [(q NN + a) 3 + c]
+    double tw[EPB][NQ][6];   // tau * w detJ (11,22,33,12,23,13)
+    KT mw[EPB][NQ];          // mu w detJ
+    TLStiff<KT, EPB, NG> k;
 };
+
+// acc += a * b for FP32 pairs (hi, lo): the product of the leading parts exactly (its rounding error by FMA), the
+// cross terms in FP32, the sum with acc.x by Knuth's TwoSum (about 48 bits)
+__device__ __forceinline__ void tl_df_fma(float2& acc, float2 a, float2 b) {
+    const float p = __fmul_rn(a.x, b.x);
+    const float pe = __fmaf_rn(a.x, b.x, -p);
+    const float x = __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x));
+    const float s = __fadd_rn(acc.x, p);
+    const float bv = __fsub_rn(s, acc.x);
+    const float err = __fadd_rn(__fsub_rn(acc.x, __fsub_rn(s, bv)), __fsub_rn(p, bv));
+    acc.x = s;
+    acc.y = __fadd_rn(acc.y, __fadd_rn(err, __fadd_rn(pe, x)));
+}
 
 // F^-1 and det F of a 3x3 matrix
 __device__ __forceinline__ double inv3(const double (*F)[3], double (*Fi)[3]) {
@@ -67,18 +101,16 @@ __device__ __forceinline__ double inv3(const double (*F)[3], double (*Fi)[3]) {
 }
 
 template <int NN, int NQ, typename KT, bool VIJ>
-__global__ void __launch_bounds__(kTLBlock) tl_kernel(int nEl, const int32_t* __restrict__ nodeDof,
-                                                      const double* __restrict__ geo, const double* __restrict__ U,
-                                                      double* __restrict__ stateOut, PropsArg props,
-                                                      const double* __restrict__ propsTable,
-                                                      const int32_t* __restrict__ elemRow,
-                                                      KT* __restrict__ Kout, double* __restrict__ Pe,
-                                                      double* __restrict__ tang, int* __restrict__ flags) {
-    constexpr int TPE = (NQ <= 8) ? 8 : 32;
-    constexpr int EPB = kTLBlock / TPE;
+__global__ void __launch_bounds__(TLShared<NN, NQ, KT>::BLOCK) tl_kernel(
+    int nEl, const int32_t* __restrict__ nodeDof, const double* __restrict__ geo, const double* __restrict__ U,
+    double* __restrict__ stateOut, PropsArg props, const double* __restrict__ propsTable,
+    const int32_t* __restrict__ elemRow, KT* __restrict__ Kout, double* __restrict__ Pe, double* __restrict__ tang,
+    int* __restrict__ flags) {
+    constexpr int TPE = TLShared<NN, NQ, KT>::TPE;
+    constexpr int EPB = TLShared<NN, NQ, KT>::EPB;
     constexpr int NP = NN * (NN + 1) / 2;
     constexpr int ND = 3 * NN;
-    constexpr int NG = 3 * NN + 1;
+    constexpr int NG0 = 3 * NN + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TLShared<NN, NQ, KT>& sh = *reinterpret_cast<TLShared<NN, NQ, KT>*>(smem_raw);
     const int tid = threadIdx.x;
@@ -99,15 +131,10 @@ __global__ void __launch_bounds__(kTLBlock) tl_kernel(int nEl, const int32_t* __
     // ---- Gauss-point phase: F, material, spatial gradients ------------------------------------
     if (valid && lane < NQ) {
         const int q = lane;
-        const double* gq = geo + ((int64_t)e * NQ + q) * NG;
+        const double* gq = geo + ((int64_t)e * NQ + q) * NG0;
         double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
         for (int a = 0; a < NN; ++a) {
-            double ga[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                ga[c] = gq[3 * a + c];
-                sh.g0[le][q][a][c] = ga[c];
-            }
+            const double ga[3] = {gq[3 * a], gq[3 * a + 1], gq[3 * a + 2]};
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -154,13 +181,30 @@ __global__ void __launch_bounds__(kTLBlock) tl_kernel(int nEl, const int32_t* __
         stateOut[12 * nQPtot + qi] = W;
 #pragma unroll
         for (int i = 0; i < 6; ++i) sh.tw[le][q][i] = tau[i] * wdet;
-        sh.sc[le][q][0] = (KT)(mu * wdet);
-        sh.sc[le][q][1] = (KT)(mb * wdet);
-        sh.sc[le][q][2] = (KT)(lb * wdet);
+        const double mbw = mb * wdet, lbw = lb * wdet;
+        sh.mw[le][q] = (KT)(mu * wdet);
+#pragma unroll 2
         for (int a = 0; a < NN; ++a) {
-            const double* g0 = sh.g0[le][q][a];
+            const double g0[3] = {gq[3 * a], gq[3 * a + 1], gq[3 * a + 2]};
+            const int at = (q * NN + a) * 3;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) sh.g[le][q][a][i] = Fi[0][i] * g0[0] + Fi[1][i] * g0[1] + Fi[2][i] * g0[2];
+            for (int i = 0; i < 3; ++i) {
+                const double gi = Fi[0][i] * g0[0] + Fi[1][i] * g0[1] + Fi[2][i] * g0[2];
+                sh.g[le][at + i] = gi;
+                if constexpr (sizeof(KT) == 8) {
+                    sh.k.g0[le][at + i] = g0[i];
+                    sh.k.gm[le][at + i] = mbw * gi;
+                    sh.k.gl[le][at + i] = lbw * gi;
+                } else {
+                    const float f = (float)gi;
+                    uint32_t hi, lo;  // split by integer operations, off the FP64 pipe
+                    split_bits((uint64_t)__double_as_longlong(g0[i]), &hi, &lo);
+                    sh.k.g0[le][at + i] = make_float2(__uint_as_float(hi), __uint_as_float(lo));
+                    sh.k.ga[le][at + i] = f;
+                    sh.k.gm[le][at + i] = (float)mbw * f;
+                    sh.k.gl[le][at + i] = (float)lbw * f;
+                }
+            }
         }
         if (tang) {
             // FP64 tangent data of this Gauss point for the matrix-free refinement residual
@@ -181,10 +225,11 @@ __global__ void __launch_bounds__(kTLBlock) tl_kernel(int nEl, const int32_t* __
         double f0 = 0, f1 = 0, f2 = 0;
         for (int q = 0; q < NQ; ++q) {
             const double* t = sh.tw[le][q];
-            const double gx = sh.g[le][q][a][0], gy = sh.g[le][q][a][1], gz = sh.g[le][q][a][2];
-            f0 += t[0] * gx + t[3] * gy + t[5] * gz;
-            f1 += t[3] * gx + t[1] * gy + t[4] * gz;
-            f2 += t[5] * gx + t[4] * gy + t[2] * gz;
+            const double* g = &sh.g[le][(q * NN + a) * 3];
+            const double gx = g[0], gy = g[1], gz = g[2];
+            f0 = fma(t[5], gz, fma(t[3], gy, fma(t[0], gx, f0)));
+            f1 = fma(t[4], gz, fma(t[1], gy, fma(t[3], gx, f1)));
+            f2 = fma(t[2], gz, fma(t[4], gy, fma(t[5], gx, f2)));
         }
         double* pe = Pe + (int64_t)e * ND + 3 * a;
         pe[0] = -f0;
@@ -192,26 +237,43 @@ __global__ void __launch_bounds__(kTLBlock) tl_kernel(int nEl, const int32_t* __
         pe[2] = -f2;
     }
 
-    // ---- stiffness blocks a <= b ---------------------------------------------------------------
+    // ---- stiffness blocks a <= b: sum_q mu w (g0_a . g0_b) I + ga (x) (mb w gb) - (lb w gb) (x) ga -------
+    // The FP64 pipe (two lanes per SM and cycle) bounds it.  FP64: 22 instructions per pair and Gauss point (40
+    // with the factors applied per pair); FP32: none, where the conversions of both gradients and the dot
+    // product took ten of the FP64 pipe per pair and point.  Hex20, 27 points: 546 elements FP64 302 -> 194 us, 3,375
+    // elements FP32 568 -> 301 us; hex8, 3,375 elements FP32 61 -> 33 us.
     for (int p = lane; p < NP; p += TPE) {
         const int a = tl_pair_a(p, NN);
         const int b = a + (p - (a * NN - a * (a - 1) / 2));
         KT k[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        KT s = 0;
         for (int q = 0; q < NQ; ++q) {
-            const KT mw = sh.sc[le][q][0], mbw = sh.sc[le][q][1], lbw = sh.sc[le][q][2];
-            const double* g0a = sh.g0[le][q][a];
-            const double* g0b = sh.g0[le][q][b];
-            const KT d0 = (KT)(g0a[0] * g0b[0] + g0a[1] * g0b[1] + g0a[2] * g0b[2]);
-            const KT ga[3] = {(KT)sh.g[le][q][a][0], (KT)sh.g[le][q][a][1], (KT)sh.g[le][q][a][2]};
-            const KT gb[3] = {(KT)sh.g[le][q][b][0], (KT)sh.g[le][q][b][1], (KT)sh.g[le][q][b][2]};
-            const KT s = mw * d0;
+            const int ia = (q * NN + a) * 3, ib = (q * NN + b) * 3;
+            KT d0, ga[3];
+            if constexpr (sizeof(KT) == 8) {
+                const double *x = &sh.k.g0[le][ia], *y = &sh.k.g0[le][ib];
+                d0 = fma(x[2], y[2], fma(x[1], y[1], x[0] * y[0]));
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ga[i] = sh.g[le][ia + i];
+            } else {
+                float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    tl_df_fma(acc, sh.k.g0[le][ia + i], sh.k.g0[le][ib + i]);
+                    ga[i] = sh.k.ga[le][ia + i];
+                }
+                d0 = acc.x + acc.y;
+            }
+            s = fma(sh.mw[le][q], d0, s);
+            const KT gm[3] = {sh.k.gm[le][ib], sh.k.gm[le][ib + 1], sh.k.gm[le][ib + 2]};
+            const KT gl[3] = {sh.k.gl[le][ib], sh.k.gl[le][ib + 1], sh.k.gl[le][ib + 2]};
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
-                for (int j = 0; j < 3; ++j) k[i][j] += mbw * ga[i] * gb[j] - lbw * gb[i] * ga[j];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) k[i][i] += s;
+                for (int j = 0; j < 3; ++j) k[i][j] = fma(-gl[i], ga[j], fma(ga[i], gm[j], k[i][j]));
         }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) k[i][i] += s;
         if (VIJ) {
             KT* ke = Kout + (int64_t)e * ND * ND;
 #pragma unroll
@@ -238,8 +300,7 @@ struct TLApplyShared {
     static constexpr int TPE = (NQ <= 8) ? 8 : 32;
     static constexpr int EPB = kTLBlock / TPE;
     double xv[EPB][NN][3];
-    double A[EPB][NQ][9];   // per Gauss point: mu w Hx
-    double Bm[EPB][NQ][9];  // per Gauss point: mb w tr(F^-1 Hx) F^-T - lb w F^-T Hx^T F^-T
+    double A[EPB][NQ][9];  // per Gauss point: mu w Hx + mb w tr(F^-1 Hx) F^-T - lb w F^-T Hx^T F^-T
 };
 
 template <int NN, int NQ>
@@ -290,8 +351,7 @@ __global__ void __launch_bounds__(kTLBlock) tl_apply_kernel(int nEl, const int32
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j) tr += Fi[i][j] * Hx[j][i];
-        // y_a = A g0_a + Bm g0_a with A = mu w Hx and, since g_a = F^-T g0_a,
-        // Bm = (mb w tr) F^-T - lb w F^-T Hx^T F^-T
+        // y_a = A g0_a with, since g_a = F^-T g0_a, A = mu w Hx + (mb w tr) F^-T - lb w F^-T Hx^T F^-T
         double M[3][3];  // Hx^T F^-T
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -301,9 +361,8 @@ __global__ void __launch_bounds__(kTLBlock) tl_apply_kernel(int nEl, const int32
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                sh.A[le][q][3 * i + j] = mw * Hx[i][j];
                 const double fm = Fi[0][i] * M[0][j] + Fi[1][i] * M[1][j] + Fi[2][i] * M[2][j];
-                sh.Bm[le][q][3 * i + j] = mbw * tr * Fi[j][i] - lbw * fm;
+                sh.A[le][q][3 * i + j] = mw * Hx[i][j] + (mbw * tr * Fi[j][i] - lbw * fm);
             }
     }
     __syncthreads();
@@ -314,10 +373,9 @@ __global__ void __launch_bounds__(kTLBlock) tl_apply_kernel(int nEl, const int32
             const double* gq = geo + ((int64_t)e * NQ + q) * NG + 3 * a;
             const double g0 = gq[0], g1 = gq[1], g2 = gq[2];
             const double* A = sh.A[le][q];
-            const double* Bm = sh.Bm[le][q];
-            y0 += (A[0] + Bm[0]) * g0 + (A[1] + Bm[1]) * g1 + (A[2] + Bm[2]) * g2;
-            y1 += (A[3] + Bm[3]) * g0 + (A[4] + Bm[4]) * g1 + (A[5] + Bm[5]) * g2;
-            y2 += (A[6] + Bm[6]) * g0 + (A[7] + Bm[7]) * g1 + (A[8] + Bm[8]) * g2;
+            y0 = fma(A[2], g2, fma(A[1], g1, fma(A[0], g0, y0)));
+            y1 = fma(A[5], g2, fma(A[4], g1, fma(A[3], g0, y1)));
+            y2 = fma(A[8], g2, fma(A[7], g1, fma(A[6], g0, y2)));
         }
         double* o = ye + (int64_t)e * ND + 3 * a;
         o[0] = y0;
@@ -340,12 +398,12 @@ static ef_status launch_tl(const Group& g, const double* U, void* K, int vij, do
     if (vij) {
         auto k = tl_kernel<NN, NQ, KT, true>;
         EF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kTLBlock, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geo, U, sOut, pa, g.propsTable, g.elemRow,
+        k<<<grid, TLShared<NN, NQ, KT>::BLOCK, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geo, U, sOut, pa, g.propsTable, g.elemRow,
                                                     (KT*)K, Pe, tang, flags);
     } else {
         auto k = tl_kernel<NN, NQ, KT, false>;
         EF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kTLBlock, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geo, U, sOut, pa, g.propsTable, g.elemRow,
+        k<<<grid, TLShared<NN, NQ, KT>::BLOCK, smem, ef::counted(s)>>>(g.nEl, g.nodeDof, g.geo, U, sOut, pa, g.propsTable, g.elemRow,
                                                     (KT*)K, Pe, tang, flags);
     }
     EF_CUDA(cudaGetLastError());
