@@ -192,11 +192,11 @@ ef_status ef_launch_newton_check(int64_t n, const double* P, const double* PExt,
 ef_status ef_launch_newton_first(int64_t n, const double* P, const double* PExt, int64_t nDir, const int64_t* dofs,
                                  const double* values, double* R, cudaStream_t s);
 ef_status ef_launch_sell_refresh(int64_t nE, const int32_t* src, const float* bsr, float* v9, void* v8, void* v1,
-                                 const int32_t* col, const float* binv, const uint8_t* mask, cudaStream_t s);
+                                 const int32_t* col, const float* binv, const uint8_t* mask, int diaN, cudaStream_t s);
 ef_status ef_launch_sell_spmv3(int nN, int nSlices, const int64_t* off, const int32_t* perm, const int32_t* col,
                                const float* v9, const float* x, const uint8_t* mask, float* y, float* xcopy, int split,
                                cudaStream_t s, const float* scale = nullptr, const int32_t* dia = nullptr,
-                               const float* binv = nullptr);
+                               int diaN = 0, const float* binv = nullptr);
 ef_status ef_launch_sell_level3_bf16(int nN, int nSlices, const int64_t* off, const int32_t* perm, const int32_t* col,
                                      const void* v8, const void* v1, const float* x, const float* r,
                                      const uint8_t* mask, float* t, const float* binv, float omega, int split,

@@ -137,6 +137,10 @@ static ef_status sell_build(ef_ctx* c) {
                 dia.insert(it, d);
             }
         if (ok && (double)32 * nS * dia.size() > 1.15 * nb) ok = false;
+        // the product reads the blocks below the diagonal as transposes of those above: the offsets come in pairs
+        for (size_t j = 0; ok && j < dia.size(); ++j)
+            if (dia[j] != -dia[dia.size() - 1 - j]) ok = false;
+        if (dia.size() % 2 == 0) ok = false;
         // each row's columns ascending (the slot order must be the row's block order)
         for (int m = 0; ok && m < n0; ++m)
             for (int32_t k = rp[m] + 1; k < rp[m + 1]; ++k)
@@ -196,10 +200,14 @@ static ef_status sell_build(ef_ctx* c) {
     EF_CHECK(upload(&c->dSellSrc, src));
     if (!perm.empty()) EF_CHECK(upload(&c->dSellPerm, perm));
     if (!dia.empty()) {
+        // the product from half the matrix gains from eight warps at any size (an iteration at 169,781 nodes 141.3 ->
+        // 137.9 us)
+        if (!getenv("EF_SELL_SPLIT_PRODUCT")) c->sellSplitProduct = std::max(c->sellSplitProduct, 8);
         EF_CHECK(upload(&c->dSellDia, dia));
         c->sellDiaN = (int)dia.size();
     }
-    c->dSellV9 = dalloc<float>(9 * (size_t)nE, &st);
+    // the FP32 planes: all slots, or in the diagonal form the diagonals from the middle one (offset 0) on
+    c->dSellV9 = dalloc<float>(dia.empty() ? 9 * (size_t)nE : 288 * (size_t)nS * (dia.size() / 2 + 1), &st);
     if (!c->dSellV9) return st;
     if (c->amgBf16) {
         c->dSellV8 = dalloc<uint4>((size_t)nE, &st);
@@ -219,7 +227,7 @@ ef_status sell_refresh(ef_ctx* c, cudaStream_t s) {
     if (c->sellMode != 1 || !c->sellStale) return EF_OK;
     EF_CHECK(ef_launch_sell_refresh(c->sellE, c->dSellSrc, (const float*)c->dBsrVals, c->dSellV9, c->dSellV8,
                                     c->dSellV1, c->dSellCol, c->sellScaled ? (const float*)c->dBinv : nullptr,
-                                    c->dMask, s));
+                                    c->dMask, c->dSellDia ? c->sellDiaN : 0, s));
     c->sellStale = false;
     return EF_OK;
 }
@@ -810,7 +818,7 @@ static ef_status amg_power(ef_ctx* c, int l, cudaStream_t s) {
         if (it + 1 == kPowerSteps) break;
         if (sellStep) {
             EF_CHECK(ef_launch_sell_spmv3(nN, c->sellSlices, c->dSellOff, c->dSellPerm, c->dSellCol, c->dSellV9, a,
-                                          mask, b, nullptr, c->sellSplitProduct, s, c->amgPowFac, c->dSellDia,
+                                          mask, b, nullptr, c->sellSplitProduct, s, c->amgPowFac, c->dSellDia, c->sellDiaN,
                                           binv));
             std::swap(a, b);
             continue;

@@ -33,10 +33,12 @@ constexpr int kSellSlicesPerCta = kSellThreads / 32;  // the product: a warp per
 // FP32 planes of K; the BF16 copy holds K, or with binv the blocks of K (M D^-1) (the block
 // inverse of the slot's column node with the rows of masked DOFs zeroed), for the residual of the
 // block-Jacobi sweep from zero: r - K (w M D^-1 r) = r - w (K M D^-1) r
+// diaN > 0 (diagonal form): the FP32 planes hold only the diagonals from the middle one on (see
+// sell_spmv3_dia_kernel)
 __global__ void sell_refresh_kernel(int64_t nE, const int32_t* __restrict__ src, const float* __restrict__ bsr,
                                     float* __restrict__ v9, uint4* __restrict__ v8, __nv_bfloat16* __restrict__ v1,
                                     const int32_t* __restrict__ col, const float* __restrict__ binv,
-                                    const uint8_t* __restrict__ mask) {
+                                    const uint8_t* __restrict__ mask, int diaN) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nE) return;
     const int64_t b = src[t];
@@ -49,9 +51,18 @@ __global__ void sell_refresh_kernel(int64_t nE, const int32_t* __restrict__ src,
         for (int k = 0; k < 9; ++k) a[k] = 0.f;
     }
     const int64_t i = t & 31;
-    float* d = v9 + 9 * (t - i) + i;
+    if (diaN == 0) {
+        float* d = v9 + 9 * (t - i) + i;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) d[32 * k] = a[k];
+        for (int k = 0; k < 9; ++k) d[32 * k] = a[k];
+    } else {
+        const int sl = (int)(t >> 5) / diaN, j = (int)(t >> 5) - sl * diaN, h = diaN / 2;
+        if (j >= h) {
+            float* d = v9 + (int64_t)288 * ((int64_t)sl * (h + 1) + j - h) + i;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) d[32 * k] = a[k];
+        }
+    }
     if (v8 && binv) {
         const int64_t c = col[t];
         const float* D = binv + 9 * c;
@@ -133,39 +144,12 @@ __device__ __forceinline__ bool sell_combine(const SellPart& p, bool active, flo
     }
 }
 
-// y = sc K x on the free DOFs (0 on masked rows); COPY: xcopy = sc x as well; sc = *scale (1 without
-// one: the FGMRES basis vector x then carries its normalisation factor); S warps per slice
-template <bool COPY, int S, bool DIA>
-__global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
-    int nN, int nSlices, const int64_t* __restrict__ off, const int32_t* __restrict__ perm,
-    const int32_t* __restrict__ col, const float* __restrict__ v9, const float* __restrict__ x,
-    const uint8_t* __restrict__ mask, float* __restrict__ y, float* __restrict__ xcopy,
-    const float* __restrict__ scale, const int32_t* __restrict__ dia, const float* __restrict__ binv) {
-    ef::dep_entry();
-    SellPart p;
-    const bool active = sell_part<S>(nSlices, off, p);
-    float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-    if (active) {
-        const int32_t* cs = col + p.e0 + p.lane;
-        const float* vs = v9 + 9 * p.e0 + p.lane;
-        const int row = p.sl * 32 + p.lane;
-#pragma unroll 3
-        for (int j = p.j0; j < p.j1; ++j) {
-            const int c3 = 3 * (DIA ? dia_column(row, __ldg(dia + j), nN) : __ldcs(cs + 32 * j));
-            const float* vv = vs + 288 * j;
-            const float a0 = __ldcs(vv), a1 = __ldcs(vv + 32), a2 = __ldcs(vv + 64);
-            const float a3 = __ldcs(vv + 96), a4 = __ldcs(vv + 128), a5 = __ldcs(vv + 160);
-            const float a6 = __ldcs(vv + 192), a7 = __ldcs(vv + 224), a8 = __ldcs(vv + 256);
-            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
-            y0 += a0 * x0 + a1 * x1 + a2 * x2;
-            y1 += a3 * x0 + a4 * x1 + a5 * x2;
-            y2 += a6 * x0 + a7 * x1 + a8 * x2;
-        }
-    }
-    if (!sell_combine<S>(p, active, y0, y1, y2)) return;
-    const int r = p.sl * 32 + p.lane;
-    if (r >= nN) return;
-    const int m = perm ? perm[r] : r;
+// the end of a product's row m: the scale, the copy of x, the mask and, with binv, D^-1
+template <bool COPY>
+__device__ __forceinline__ void sell_product_end(int m, const float* __restrict__ x, const uint8_t* __restrict__ mask,
+                                                 float* __restrict__ y, float* __restrict__ xcopy,
+                                                 const float* __restrict__ scale, const float* __restrict__ binv, float y0,
+                                                 float y1, float y2) {
     const int d = 3 * m;
     if (scale) {
         const float sc = *scale;
@@ -197,6 +181,102 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
     y[d + 0] = y0;
     y[d + 1] = y1;
     y[d + 2] = y2;
+}
+
+// y = sc K x on the free DOFs (0 on masked rows); COPY: xcopy = sc x as well; sc = *scale (1 without
+// one: the FGMRES basis vector x then carries its normalisation factor); S warps per slice
+template <bool COPY, int S>
+__global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
+    int nN, int nSlices, const int64_t* __restrict__ off, const int32_t* __restrict__ perm,
+    const int32_t* __restrict__ col, const float* __restrict__ v9, const float* __restrict__ x,
+    const uint8_t* __restrict__ mask, float* __restrict__ y, float* __restrict__ xcopy,
+    const float* __restrict__ scale, const float* __restrict__ binv) {
+    ef::dep_entry();
+    SellPart p;
+    const bool active = sell_part<S>(nSlices, off, p);
+    float y0 = 0.f, y1 = 0.f, y2 = 0.f;
+    if (active) {
+        const int32_t* cs = col + p.e0 + p.lane;
+        const float* vs = v9 + 9 * p.e0 + p.lane;
+#pragma unroll 3
+        for (int j = p.j0; j < p.j1; ++j) {
+            const int c3 = 3 * __ldcs(cs + 32 * j);
+            const float* vv = vs + 288 * j;
+            const float a0 = __ldcs(vv), a1 = __ldcs(vv + 32), a2 = __ldcs(vv + 64);
+            const float a3 = __ldcs(vv + 96), a4 = __ldcs(vv + 128), a5 = __ldcs(vv + 160);
+            const float a6 = __ldcs(vv + 192), a7 = __ldcs(vv + 224), a8 = __ldcs(vv + 256);
+            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
+            y0 += a0 * x0 + a1 * x1 + a2 * x2;
+            y1 += a3 * x0 + a4 * x1 + a5 * x2;
+            y2 += a6 * x0 + a7 * x1 + a8 * x2;
+        }
+    }
+    if (!sell_combine<S>(p, active, y0, y1, y2)) return;
+    const int r = p.sl * 32 + p.lane;
+    if (r >= nN) return;
+    sell_product_end<COPY>(perm ? perm[r] : r, x, mask, y, xcopy, scale, binv, y0, y1, y2);
+}
+
+// The product in the diagonal form from half the matrix.  K is symmetric to the bit (both blocks of a pair of
+// nodes sum the same element blocks in the same order), so only the diagonals j >= diaN / 2 are stored: the block of
+// diagonal -d in row r is the transpose of the one of diagonal d in row r - d, which the rows a little
+// further up have just brought into L1 and L2.  The order of a row's sums is the full form's: the same bits.
+// What bounds the product is HBM (the full form's 165 MB at 169,781 nodes); half the values leave it
+// 86 MB of them and L2 the rest.  STREAM: the blocks are marked for early eviction, above 60,000 nodes, where an
+// iteration's matrices no longer fit into L2 and would evict the basis.  us of a product, full form and now:
+// 11,849 nodes 8.3 -> 6.5, 38,125 nodes 12.7 -> 9.3, 88,209 nodes 23.0 -> 21.0, 169,781 nodes 35.8 -> 32.8 (an iteration
+// 46.8 against 48.9 us without STREAM and with it at 11,849 nodes, 142 against 138 at 169,781).
+template <bool COPY, int S, bool STREAM>
+__global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_dia_kernel(
+    int nN, int nSlices, int diaN, const float* __restrict__ v9, const float* __restrict__ x,
+    const uint8_t* __restrict__ mask, float* __restrict__ y, float* __restrict__ xcopy,
+    const float* __restrict__ scale, const int32_t* __restrict__ dia, const float* __restrict__ binv) {
+    ef::dep_entry();
+    constexpr int spc = sell_split_threads(S) / (32 * S);
+    SellPart p;
+    p.lane = threadIdx.x & 31;
+    const int wi = threadIdx.x >> 5;
+    p.sl = blockIdx.x * spc + wi / S;
+    p.h = wi % S;
+    const bool active = p.sl < nSlices;
+    p.j0 = (p.h * diaN + S - 1) / S;
+    p.j1 = ((p.h + 1) * diaN + S - 1) / S;
+    const int row = p.sl * 32 + p.lane;
+    const int mid = diaN / 2, stored = mid + 1;  // diagonals of a slice
+    auto ld = [](const float* a) { return STREAM ? __ldcs(a) : *a; };
+    float y0 = 0.f, y1 = 0.f, y2 = 0.f;
+    if (active) {
+        const int jm = min(p.j1, max(p.j0, mid));
+#pragma unroll 3
+        for (int j = p.j0; j < jm; ++j) {  // below the middle: transposed from row r + dia[j] (a block of rows before 0: none)
+            const int c = row + __ldg(dia + j);
+            const int cc = min(max(c, 0), nN - 1);
+            const float* vv = v9 + (int64_t)288 * ((int64_t)(cc >> 5) * stored + (mid - j)) + (cc & 31);
+            const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
+            const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
+            const float x0 = x[3 * cc], x1 = x[3 * cc + 1], x2 = x[3 * cc + 2];
+            if (c == cc) {
+                y0 += a0 * x0 + a3 * x1 + a6 * x2;
+                y1 += a1 * x0 + a4 * x1 + a7 * x2;
+                y2 += a2 * x0 + a5 * x1 + a8 * x2;
+            }
+        }
+        const float* vs = v9 + (int64_t)288 * ((int64_t)p.sl * stored - mid) + p.lane;
+#pragma unroll 3
+        for (int j = max(p.j0, mid); j < p.j1; ++j) {
+            const int c3 = 3 * dia_column(row, __ldg(dia + j), nN);
+            const float* vv = vs + 288 * j;
+            const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
+            const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
+            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
+            y0 += a0 * x0 + a1 * x1 + a2 * x2;
+            y1 += a3 * x0 + a4 * x1 + a5 * x2;
+            y2 += a6 * x0 + a7 * x1 + a8 * x2;
+        }
+    }
+    if (!sell_combine<S>(p, active, y0, y1, y2)) return;
+    if (row >= nN) return;
+    sell_product_end<COPY>(row, x, mask, y, xcopy, scale, binv, y0, y1, y2);
 }
 
 // t = r - ys K x on the fine level (0 on masked rows), or with binv a damped block-Jacobi sweep
@@ -352,28 +432,31 @@ static inline unsigned sell_split_grid(int nSlices, int S) {
 }
 
 ef_status ef_launch_sell_refresh(int64_t nE, const int32_t* src, const float* bsr, float* v9, void* v8, void* v1,
-                                 const int32_t* col, const float* binv, const uint8_t* mask, cudaStream_t s) {
+                                 const int32_t* col, const float* binv, const uint8_t* mask, int diaN, cudaStream_t s) {
     if (nE <= 0) return EF_OK;
     sell_refresh_kernel<<<(unsigned)((nE + 255) / 256), 256, 0, ef::counted(s)>>>(
-        nE, src, bsr, v9, (uint4*)v8, (__nv_bfloat16*)v1, col, binv, mask);
+        nE, src, bsr, v9, (uint4*)v8, (__nv_bfloat16*)v1, col, binv, mask, diaN);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }
 
 ef_status ef_launch_sell_spmv3(int nN, int nSlices, const int64_t* off, const int32_t* perm, const int32_t* col,
                                const float* v9, const float* x, const uint8_t* mask, float* y, float* xcopy, int split,
-                               cudaStream_t s, const float* scale, const int32_t* dia, const float* binv) {
+                               cudaStream_t s, const float* scale, const int32_t* dia, int diaN, const float* binv) {
     if (nSlices <= 0) return EF_OK;
 #define EF_SPMV3(C_, S_)                                                                                              \
     do {                                                                                                              \
-        if (dia)                                                                                                      \
-            EF_CUDA(ef::launch_dep(sell_spmv3_kernel<C_, S_, true>, sell_split_grid(nSlices, S_),                     \
-                                   sell_split_threads(S_), 0, s, nN, nSlices, off, perm, col, v9, x, mask, y, xcopy,  \
-                                   scale, dia, binv));                                                                \
+        if (dia && nN > 60000)                                                                                        \
+            EF_CUDA(ef::launch_dep(sell_spmv3_dia_kernel<C_, S_, true>, sell_split_grid(nSlices, S_),                 \
+                                   sell_split_threads(S_), 0, s, nN, nSlices, diaN, v9, x, mask, y, xcopy, scale,     \
+                                   dia, binv));                                                                       \
+        else if (dia)                                                                                                 \
+            EF_CUDA(ef::launch_dep(sell_spmv3_dia_kernel<C_, S_, false>, sell_split_grid(nSlices, S_),                \
+                                   sell_split_threads(S_), 0, s, nN, nSlices, diaN, v9, x, mask, y, xcopy, scale,     \
+                                   dia, binv));                                                                       \
         else                                                                                                          \
-            EF_CUDA(ef::launch_dep(sell_spmv3_kernel<C_, S_, false>, sell_split_grid(nSlices, S_),                    \
-                                   sell_split_threads(S_), 0, s, nN, nSlices, off, perm, col, v9, x, mask, y, xcopy,  \
-                                   scale, dia, binv));                                                                \
+            EF_CUDA(ef::launch_dep(sell_spmv3_kernel<C_, S_>, sell_split_grid(nSlices, S_), sell_split_threads(S_),   \
+                                   0, s, nN, nSlices, off, perm, col, v9, x, mask, y, xcopy, scale, binv));           \
     } while (0)
 #define EF_SPMV3_S(C_)      \
     if (split == 2)         \
