@@ -76,10 +76,10 @@ static ef_status sell_build(ef_ctx* c) {
     };
     const int n0 = (int)c->nNodes;
     // Warps per slice: as many as it takes to give an SM enough warps to hide a step's loads, and no more (they
-    // meet in shared memory).  us of the product / the preconditioner with 4, 8 and 16 warps: 4,225 nodes 8.4 / 24.1,
-    // 8.0 / 21.4, 7.3 / 21.2; 18,081 nodes 12.6 / 37.8, 10.4 / 33.5, 9.7 / 31.2; 88,209 nodes 24.7 / 60.6,
-    // 23.0 / 59.8, 25.0 / 63.0; 169,781 nodes 35.4 / 83.6, 36.1 / 88.0, 41.3 / 101; rows of quadratic elements (up to
-    // 81 blocks) 7,500 nodes 28.5, 17.9 and 12.7 (32 warps: 10.4) for the product
+    // meet in shared memory).  us of the product / the preconditioner with 4, 8 and 16 warps: 4,225 nodes 8.5 / 23.4,
+    // 8.4 / 21.2, 6.4 / 19.3; 18,081 nodes 8.6 / 35.7, 8.4 / 31.6, 8.4 / 29.9; 38,125 nodes 10.4 / 40.0, 9.0 / 36.9,
+    // 10.5 / 38.0; 169,781 nodes 28.7 / 78.0, 26.8 / 79.9, 38.8 / 92.4; rows of quadratic elements (up to 81 blocks) at
+    // 7,412 nodes 20.7 / 38.0, 13.9 / 29.4, 10.5 / 25.3 (32 warps: the same)
     const int perSM = (n0 + 32 * c->nSM - 1) / (32 * c->nSM);  // slices
     const int warps = perSM <= 6 ? 16 : (perSM <= 24 ? 8 : 4);
     c->sellSplit = split(getenv("EF_SELL_SPLIT"), warps);
@@ -200,8 +200,8 @@ static ef_status sell_build(ef_ctx* c) {
     EF_CHECK(upload(&c->dSellSrc, src));
     if (!perm.empty()) EF_CHECK(upload(&c->dSellPerm, perm));
     if (!dia.empty()) {
-        // the product from half the matrix gains from eight warps at any size (an iteration at 169,781 nodes 141.3 ->
-        // 137.9 us)
+        // the product from half the matrix gains from eight warps at any size (at 169,781 nodes 28.7 ->
+        // 26.8 us)
         if (!getenv("EF_SELL_SPLIT_PRODUCT")) c->sellSplitProduct = std::max(c->sellSplitProduct, 8);
         EF_CHECK(upload(&c->dSellDia, dia));
         c->sellDiaN = (int)dia.size();

@@ -183,6 +183,22 @@ __device__ __forceinline__ void sell_product_end(int m, const float* __restrict_
     y[d + 2] = y2;
 }
 
+__device__ __forceinline__ void sell_block_add(const float (&a)[9], const float (&xv)[3], float& y0, float& y1, float& y2) {
+    y0 += a[0] * xv[0] + a[1] * xv[1] + a[2] * xv[2];
+    y1 += a[3] * xv[0] + a[4] * xv[1] + a[5] * xv[2];
+    y2 += a[6] * xv[0] + a[7] * xv[1] + a[8] * xv[2];
+}
+
+// The slot columns of a warp are taken two at a time, all their loads first (the second clamped to the last one and
+// left out of the sum where the count is odd): an unrolled loop falls back to one column after the other for its
+// remainder, which with a slice split over several warps is most of it.  More than two take registers from
+// the warps that hide the loads.  us before, with two and with four columns: the product at 169,781 nodes 32.8, 26.8 and
+// 26.8, of 81-block rows at 26,745 nodes 20.7, 18.5 and 19.8; the preconditioner (its residual) 82.4, 78.2 and 79.4 at
+// 169,781 nodes, 31.6, 30.0 and 33.8 at 18,081.  What bounds them then is the latency of the gathers: the 82 MB that a
+// residual of 169,781 nodes reads take 14.5 us (5.7 TB/s) by themselves; a ring of slices in shared memory kept ahead
+// by bulk copies was slower (preconditioner 100 us), as fewer warps gather.
+constexpr int kSellBatch = 2;
+
 // y = sc K x on the free DOFs (0 on masked rows); COPY: xcopy = sc x as well; sc = *scale (1 without
 // one: the FGMRES basis vector x then carries its normalisation factor); S warps per slice
 template <bool COPY, int S>
@@ -198,17 +214,20 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
     if (active) {
         const int32_t* cs = col + p.e0 + p.lane;
         const float* vs = v9 + 9 * p.e0 + p.lane;
-#pragma unroll 3
-        for (int j = p.j0; j < p.j1; ++j) {
-            const int c3 = 3 * __ldcs(cs + 32 * j);
-            const float* vv = vs + 288 * j;
-            const float a0 = __ldcs(vv), a1 = __ldcs(vv + 32), a2 = __ldcs(vv + 64);
-            const float a3 = __ldcs(vv + 96), a4 = __ldcs(vv + 128), a5 = __ldcs(vv + 160);
-            const float a6 = __ldcs(vv + 192), a7 = __ldcs(vv + 224), a8 = __ldcs(vv + 256);
-            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
-            y0 += a0 * x0 + a1 * x1 + a2 * x2;
-            y1 += a3 * x0 + a4 * x1 + a5 * x2;
-            y2 += a6 * x0 + a7 * x1 + a8 * x2;
+        for (int j = p.j0; j < p.j1; j += kSellBatch) {
+            float a[kSellBatch][9], xv[kSellBatch][3];
+#pragma unroll
+            for (int u = 0; u < kSellBatch; ++u) {
+                const int k = min(j + u, p.j1 - 1);
+                const int c3 = 3 * __ldcs(cs + 32 * k);
+#pragma unroll
+                for (int i = 0; i < 9; ++i) a[u][i] = __ldcs(vs + 288 * k + 32 * i);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) xv[u][i] = x[c3 + i];
+            }
+#pragma unroll
+            for (int u = 0; u < kSellBatch; ++u)
+                if (j + u < p.j1) sell_block_add(a[u], xv[u], y0, y1, y2);
         }
     }
     if (!sell_combine<S>(p, active, y0, y1, y2)) return;
@@ -221,11 +240,11 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
 // nodes sum the same element blocks in the same order), so only the diagonals j >= diaN / 2 are stored: the block of
 // diagonal -d in row r is the transpose of the one of diagonal d in row r - d, which the rows a little
 // further up have just brought into L1 and L2.  The order of a row's sums is the full form's: the same bits.
-// What bounds the product is HBM (the full form's 165 MB at 169,781 nodes); half the values leave it
-// 86 MB of them and L2 the rest.  STREAM: the blocks are marked for early eviction, above 60,000 nodes, where an
-// iteration's matrices no longer fit into L2 and would evict the basis.  us of a product, full form and now:
-// 11,849 nodes 8.3 -> 6.5, 38,125 nodes 12.7 -> 9.3, 88,209 nodes 23.0 -> 21.0, 169,781 nodes 35.8 -> 32.8 (an iteration
-// 46.8 against 48.9 us without STREAM and with it at 11,849 nodes, 142 against 138 at 169,781).
+// Half the values leave HBM 86 MB of them at 169,781 nodes (full form 165 MB) and L2 the rest.  STREAM (above 60,000 nodes, where
+// an iteration's matrices no longer fit into L2 and would evict the basis): the blocks are marked for early eviction
+// and taken two at a time; below, one after the other from cached lines (11,849 nodes: 6.7 us against 7.5 two at a
+// time, 38,125 nodes: 9.1 against 10.4).  us of a product, full form and now: 11,849 nodes 8.3 -> 6.7, 38,125 nodes
+// 12.7 -> 9.1, 88,209 nodes 23.0 -> 16.7, 169,781 nodes 35.8 -> 26.8.
 template <bool COPY, int S, bool STREAM>
 __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_dia_kernel(
     int nN, int nSlices, int diaN, const float* __restrict__ v9, const float* __restrict__ x,
@@ -246,37 +265,105 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_dia_kernel(
     auto ld = [](const float* a) { return STREAM ? __ldcs(a) : *a; };
     float y0 = 0.f, y1 = 0.f, y2 = 0.f;
     if (active) {
-        const int jm = min(p.j1, max(p.j0, mid));
-#pragma unroll 3
-        for (int j = p.j0; j < jm; ++j) {  // below the middle: transposed from row r + dia[j] (a block of rows before 0: none)
-            const int c = row + __ldg(dia + j);
-            const int cc = min(max(c, 0), nN - 1);
-            const float* vv = v9 + (int64_t)288 * ((int64_t)(cc >> 5) * stored + (mid - j)) + (cc & 31);
-            const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
-            const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
-            const float x0 = x[3 * cc], x1 = x[3 * cc + 1], x2 = x[3 * cc + 2];
-            if (c == cc) {
-                y0 += a0 * x0 + a3 * x1 + a6 * x2;
-                y1 += a1 * x0 + a4 * x1 + a7 * x2;
-                y2 += a2 * x0 + a5 * x1 + a8 * x2;
+        if constexpr (STREAM) {
+            for (int j = p.j0; j < p.j1; j += kSellBatch) {
+                float a[kSellBatch][9], xv[kSellBatch][3];
+                bool in[kSellBatch];
+#pragma unroll
+                for (int u = 0; u < kSellBatch; ++u) {
+                    const int k = min(j + u, p.j1 - 1);
+                    const int c = row + __ldg(dia + k), cc = min(max(c, 0), nN - 1);
+                    // below the middle: transposed from row c (a block of rows before 0: none)
+                    const bool below = k < mid;
+                    const int rr = below ? cc : row;
+                    const float* vv = v9 + (int64_t)288 * ((int64_t)(rr >> 5) * stored + (below ? mid - k : k - mid)) + (rr & 31);
+                    in[u] = j + u < p.j1 && (!below || c == cc);
+                    a[u][0] = ld(vv);
+                    a[u][1] = ld(vv + (below ? 96 : 32));
+                    a[u][2] = ld(vv + (below ? 192 : 64));
+                    a[u][3] = ld(vv + (below ? 32 : 96));
+                    a[u][4] = ld(vv + 128);
+                    a[u][5] = ld(vv + (below ? 224 : 160));
+                    a[u][6] = ld(vv + (below ? 64 : 192));
+                    a[u][7] = ld(vv + (below ? 160 : 224));
+                    a[u][8] = ld(vv + 256);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) xv[u][i] = x[3 * cc + i];
+                }
+#pragma unroll
+                for (int u = 0; u < kSellBatch; ++u)
+                    if (in[u]) sell_block_add(a[u], xv[u], y0, y1, y2);
             }
-        }
-        const float* vs = v9 + (int64_t)288 * ((int64_t)p.sl * stored - mid) + p.lane;
+        } else {
+            const int jm = min(p.j1, max(p.j0, mid));
 #pragma unroll 3
-        for (int j = max(p.j0, mid); j < p.j1; ++j) {
-            const int c3 = 3 * dia_column(row, __ldg(dia + j), nN);
-            const float* vv = vs + 288 * j;
-            const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
-            const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
-            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
-            y0 += a0 * x0 + a1 * x1 + a2 * x2;
-            y1 += a3 * x0 + a4 * x1 + a5 * x2;
-            y2 += a6 * x0 + a7 * x1 + a8 * x2;
+            for (int j = p.j0; j < jm; ++j) {  // below the middle: transposed from row r + dia[j] (a block of rows before 0: none)
+                const int c = row + __ldg(dia + j);
+                const int cc = min(max(c, 0), nN - 1);
+                const float* vv = v9 + (int64_t)288 * ((int64_t)(cc >> 5) * stored + (mid - j)) + (cc & 31);
+                const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
+                const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
+                const float x0 = x[3 * cc], x1 = x[3 * cc + 1], x2 = x[3 * cc + 2];
+                if (c == cc) {
+                    y0 += a0 * x0 + a3 * x1 + a6 * x2;
+                    y1 += a1 * x0 + a4 * x1 + a7 * x2;
+                    y2 += a2 * x0 + a5 * x1 + a8 * x2;
+                }
+            }
+            const float* vs = v9 + (int64_t)288 * ((int64_t)p.sl * stored - mid) + p.lane;
+#pragma unroll 3
+            for (int j = max(p.j0, mid); j < p.j1; ++j) {
+                const int c3 = 3 * dia_column(row, __ldg(dia + j), nN);
+                const float* vv = vs + 288 * j;
+                const float a0 = ld(vv), a1 = ld(vv + 32), a2 = ld(vv + 64), a3 = ld(vv + 96), a4 = ld(vv + 128);
+                const float a5 = ld(vv + 160), a6 = ld(vv + 192), a7 = ld(vv + 224), a8 = ld(vv + 256);
+                const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
+                y0 += a0 * x0 + a1 * x1 + a2 * x2;
+                y1 += a3 * x0 + a4 * x1 + a5 * x2;
+                y2 += a6 * x0 + a7 * x1 + a8 * x2;
+            }
         }
     }
     if (!sell_combine<S>(p, active, y0, y1, y2)) return;
     if (row >= nN) return;
     sell_product_end<COPY>(row, x, mask, y, xcopy, scale, binv, y0, y1, y2);
+}
+
+// y += one BF16 block times x (values 0..7 in q, value 8 in b8)
+__device__ __forceinline__ void sell_bf16_step(const uint4& q, __nv_bfloat16 b8, float x0, float x1, float x2, float& y0,
+                                               float& y1, float& y2) {
+    const float w8 = __bfloat162float(b8);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+    const float2 a01 = __bfloat1622float2(h[0]), a23 = __bfloat1622float2(h[1]);
+    const float2 a45 = __bfloat1622float2(h[2]), a67 = __bfloat1622float2(h[3]);
+    y0 += a01.x * x0 + a01.y * x1 + a23.x * x2;
+    y1 += a23.y * x0 + a45.x * x1 + a45.y * x2;
+    y2 += a67.x * x0 + a67.y * x1 + w8 * x2;
+}
+
+// the end of a row m of sell_level3_bf16_kernel: K x = (y0, y1, y2)
+__device__ __forceinline__ void sell_level3_end(int m, const float* __restrict__ x, const float* __restrict__ r,
+                                                const uint8_t* __restrict__ mask, float* __restrict__ t,
+                                                const float* __restrict__ binv, float omega, float ys, float y0, float y1,
+                                                float y2) {
+    const int d = 3 * m;
+    const bool k0 = mask[d], k1 = mask[d + 1], k2 = mask[d + 2];
+    const float t0 = k0 ? 0.f : r[d] - ys * y0, t1 = k1 ? 0.f : r[d + 1] - ys * y1,
+                t2 = k2 ? 0.f : r[d + 2] - ys * y2;
+    if (!binv) {
+        t[d] = t0;
+        t[d + 1] = t1;
+        t[d + 2] = t2;
+        return;
+    }
+    const float* B = binv + 9 * (int64_t)m;
+    const float z0 = B[0] * t0 + B[1] * t1 + B[2] * t2;
+    const float z1 = B[3] * t0 + B[4] * t1 + B[5] * t2;
+    const float z2 = B[6] * t0 + B[7] * t1 + B[8] * t2;
+    const float x0 = x[d], x1 = x[d + 1], x2 = x[d + 2];
+    t[d] = k0 ? x0 : x0 + omega * z0;
+    t[d + 1] = k1 ? x1 : x1 + omega * z1;
+    t[d + 2] = k2 ? x2 : x2 + omega * z2;
 }
 
 // t = r - ys K x on the fine level (0 on masked rows), or with binv a damped block-Jacobi sweep
@@ -296,42 +383,29 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_level3_bf16_kernel
         const uint4* qs = v8 + p.e0 + p.lane;
         const __nv_bfloat16* ws = v1 + p.e0 + p.lane;
         const int row = p.sl * 32 + p.lane;
-#pragma unroll 4
-        for (int j = p.j0; j < p.j1; ++j) {
-            const int c3 = 3 * (DIA ? dia_column(row, __ldg(dia + j), nN) : __ldcs(cs + 32 * j));
-            const uint4 q = __ldcs(qs + 32 * j);
-            const float w8 = __bfloat162float(ws[32 * j]);
-            const float x0 = x[c3], x1 = x[c3 + 1], x2 = x[c3 + 2];
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-            const float2 a01 = __bfloat1622float2(h[0]), a23 = __bfloat1622float2(h[1]);
-            const float2 a45 = __bfloat1622float2(h[2]), a67 = __bfloat1622float2(h[3]);
-            y0 += a01.x * x0 + a01.y * x1 + a23.x * x2;
-            y1 += a23.y * x0 + a45.x * x1 + a45.y * x2;
-            y2 += a67.x * x0 + a67.y * x1 + w8 * x2;
+        for (int j = p.j0; j < p.j1; j += kSellBatch) {
+            uint4 q[kSellBatch];
+            __nv_bfloat16 b8[kSellBatch];
+            float xv[kSellBatch][3];
+#pragma unroll
+            for (int u = 0; u < kSellBatch; ++u) {
+                const int k = min(j + u, p.j1 - 1);
+                const int c3 = 3 * (DIA ? dia_column(row, __ldg(dia + k), nN) : __ldcs(cs + 32 * k));
+                q[u] = __ldcs(qs + 32 * k);
+                b8[u] = ws[32 * k];
+                xv[u][0] = x[c3];
+                xv[u][1] = x[c3 + 1];
+                xv[u][2] = x[c3 + 2];
+            }
+#pragma unroll
+            for (int u = 0; u < kSellBatch; ++u)
+                if (j + u < p.j1) sell_bf16_step(q[u], b8[u], xv[u][0], xv[u][1], xv[u][2], y0, y1, y2);
         }
     }
     if (!sell_combine<S>(p, active, y0, y1, y2)) return;
     const int rr = p.sl * 32 + p.lane;
     if (rr >= nN) return;
-    const int m = perm ? perm[rr] : rr;
-    const int d = 3 * m;
-    const bool k0 = mask[d], k1 = mask[d + 1], k2 = mask[d + 2];
-    const float t0 = k0 ? 0.f : r[d] - ys * y0, t1 = k1 ? 0.f : r[d + 1] - ys * y1,
-                t2 = k2 ? 0.f : r[d + 2] - ys * y2;
-    if (!binv) {
-        t[d] = t0;
-        t[d + 1] = t1;
-        t[d + 2] = t2;
-        return;
-    }
-    const float* B = binv + 9 * (int64_t)m;
-    const float z0 = B[0] * t0 + B[1] * t1 + B[2] * t2;
-    const float z1 = B[3] * t0 + B[4] * t1 + B[5] * t2;
-    const float z2 = B[6] * t0 + B[7] * t1 + B[8] * t2;
-    const float x0 = x[d], x1 = x[d + 1], x2 = x[d + 2];
-    t[d] = k0 ? x0 : x0 + omega * z0;
-    t[d + 1] = k1 ? x1 : x1 + omega * z1;
-    t[d + 2] = k2 ? x2 : x2 + omega * z2;
+    sell_level3_end(perm ? perm[rr] : rr, x, r, mask, t, binv, omega, ys, y0, y1, y2);
 }
 
 // ---- fused fine-level post-smoothing x = w D^-1 (r + t) + C e (amg_sa_body.h) ----------------
@@ -373,6 +447,33 @@ __device__ __forceinline__ float2 bf16x2_floats(uint32_t v) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
 }
 
+// y += C e of one block
+__device__ __forceinline__ void sa_post_step(const float* ev, const uint4& u, const uint4& v, uint32_t w2,
+                                             float& y0, float& y1, float& y2) {
+    const float e0 = ev[0], e1 = ev[1], e2 = ev[2], e3 = ev[3], e4 = ev[4], e5 = ev[5];
+    const float2 c01 = bf16x2_floats(u.x), c23 = bf16x2_floats(u.y), c45 = bf16x2_floats(u.z);
+    const float2 c67 = bf16x2_floats(u.w), c89 = bf16x2_floats(v.x), cab = bf16x2_floats(v.y);
+    const float2 ccd = bf16x2_floats(v.z), cef = bf16x2_floats(v.w), cgh = bf16x2_floats(w2);
+    y0 += c01.x * e0 + c01.y * e1 + c23.x * e2 + c23.y * e3 + c45.x * e4 + c45.y * e5;
+    y1 += c67.x * e0 + c67.y * e1 + c89.x * e2 + c89.y * e3 + cab.x * e4 + cab.y * e5;
+    y2 += ccd.x * e0 + ccd.y * e1 + cef.x * e2 + cef.y * e3 + cgh.x * e4 + cgh.y * e5;
+}
+
+// the end of row m: x = w D^-1 (r + t) + y
+__device__ __forceinline__ void sa_post_end(int m, const float* __restrict__ r, const float* __restrict__ t,
+                                            const float* __restrict__ binv, const uint8_t* __restrict__ mask, float omega,
+                                            float* __restrict__ x, float y0, float y1, float y2) {
+    const int d = 3 * m;
+    const float s0 = r[d] + t[d], s1 = r[d + 1] + t[d + 1], s2 = r[d + 2] + t[d + 2];
+    const float* B = binv + 9 * (int64_t)m;
+    const float z0 = B[0] * s0 + B[1] * s1 + B[2] * s2;
+    const float z1 = B[3] * s0 + B[4] * s1 + B[5] * s2;
+    const float z2 = B[6] * s0 + B[7] * s1 + B[8] * s2;
+    x[d] = mask[d] ? 0.f : omega * z0 + y0;
+    x[d + 1] = mask[d + 1] ? 0.f : omega * z1 + y1;
+    x[d + 2] = mask[d + 2] ? 0.f : omega * z2 + y2;
+}
+
 // x = w D^-1 (r + t) + sum over the row's C blocks of C e[col] (masked DOFs 0); S warps per slice
 template <int S>
 __global__ void __launch_bounds__(sell_split_threads(S)) sa_post_fused_kernel(
@@ -393,30 +494,13 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sa_post_fused_kernel(
 #pragma unroll 2
         for (int j = p.j0; j < p.j1; ++j) {
             const float* ev = e + 6 * (int64_t)__ldcs(cs + 32 * j);
-            const uint4 u = __ldcs(a0 + 32 * j), v = __ldcs(a1 + 32 * j);
-            const uint32_t w2 = __ldcs(a2 + 32 * j);
-            const float e0 = ev[0], e1 = ev[1], e2 = ev[2], e3 = ev[3], e4 = ev[4], e5 = ev[5];
-            const float2 c01 = bf16x2_floats(u.x), c23 = bf16x2_floats(u.y), c45 = bf16x2_floats(u.z);
-            const float2 c67 = bf16x2_floats(u.w), c89 = bf16x2_floats(v.x), cab = bf16x2_floats(v.y);
-            const float2 ccd = bf16x2_floats(v.z), cef = bf16x2_floats(v.w), cgh = bf16x2_floats(w2);
-            y0 += c01.x * e0 + c01.y * e1 + c23.x * e2 + c23.y * e3 + c45.x * e4 + c45.y * e5;
-            y1 += c67.x * e0 + c67.y * e1 + c89.x * e2 + c89.y * e3 + cab.x * e4 + cab.y * e5;
-            y2 += ccd.x * e0 + ccd.y * e1 + cef.x * e2 + cef.y * e3 + cgh.x * e4 + cgh.y * e5;
+            sa_post_step(ev, __ldcs(a0 + 32 * j), __ldcs(a1 + 32 * j), __ldcs(a2 + 32 * j), y0, y1, y2);
         }
     }
     if (!sell_combine<S>(p, active, y0, y1, y2)) return;
     const int rr = p.sl * 32 + p.lane;
     if (rr >= nN) return;
-    const int m = perm ? perm[rr] : rr;
-    const int d = 3 * m;
-    const float s0 = r[d] + t[d], s1 = r[d + 1] + t[d + 1], s2 = r[d + 2] + t[d + 2];
-    const float* B = binv + 9 * (int64_t)m;
-    const float z0 = B[0] * s0 + B[1] * s1 + B[2] * s2;
-    const float z1 = B[3] * s0 + B[4] * s1 + B[5] * s2;
-    const float z2 = B[6] * s0 + B[7] * s1 + B[8] * s2;
-    x[d] = mask[d] ? 0.f : omega * z0 + y0;
-    x[d + 1] = mask[d + 1] ? 0.f : omega * z1 + y1;
-    x[d + 2] = mask[d + 2] ? 0.f : omega * z2 + y2;
+    sa_post_end(perm ? perm[rr] : rr, r, t, binv, mask, omega, x, y0, y1, y2);
 }
 
 }  // namespace ef
