@@ -177,8 +177,9 @@ __device__ __forceinline__ double flip_sign(double x, int neg) {
 template <int NN, int NQ, typename KT>
 struct SSShared {
     static constexpr int TPE = (NQ <= 8) ? 8 : 32;
-    // two elements a CTA for the FP64 stiffness of up to 27 Gauss points, whose scratch is twice as large
-    static constexpr int BLOCK = (TPE == 32 && sizeof(KT) == 8) ? 64 : kBlock;
+    // FP64: small CTAs (8 elements of 8 Gauss points, 2 of 27, whose scratch is twice as large), which deal the FP64 pipe's
+    // work out evenly over the SMs where an SM gets few elements (2,500 hex8: 113 -> 93 us with 4 or 8 of them for 16)
+    static constexpr int BLOCK = sizeof(KT) == 8 ? 64 : kBlock;
     static constexpr int EPB = BLOCK / TPE;
     static constexpr int NG = NQ * NN * 3 + 1;
     // per-element rows padded by one entry, so that the elements of a warp fall on different banks
@@ -196,7 +197,7 @@ struct SSShared {
 
 // Element loop of one group: strain increment, constitutive update, Pe (FP64) and Ke blocks (KT).
 template <int NN, int NQ, typename KT, int MAT, bool VIJ>
-__global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ? (NQ <= 8 ? 3 : 4) : 5) small_strain_kernel(
+__global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ? (NQ <= 8 ? 6 : 4) : 5) small_strain_kernel(
     int nEl, const int32_t* __restrict__ nodeDof, const float2* __restrict__ geoS, const double* __restrict__ geo,
     const double* __restrict__ dU,
     const double* __restrict__ stateIn, double* __restrict__ stateOut, PropsArg props,
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
         pe[2] = -df_value_sel(f2, intConv);
     }
 
-    auto store = [&](int p, int a, int b, const KT (&k)[3][3]) {
+    auto store = [&](int e, int p, int a, int b, const KT (&k)[3][3]) {
         if (VIJ) {
             // reference VIJ layout: value a*n+b of the element slice holds Ke[a][b]
             KT* ke = Kout + (int64_t)e * ND * ND;
@@ -351,21 +352,33 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
                 for (int j = 0; j < 3; ++j) kb[i * 3 + j] = k[i][j];
         }
     };
+    // the pairs of nodes of the CTA's elements, dealt out over all threads: a warp has those of one or two elements (the
+    // plastic branch is then rarely taken for some of its lanes only) and 36 pairs an element leave no lanes idle (10,240
+    // hex8 J2 elements in FP64 312 -> 292 us, 160,000 in FP32, where the FP64 constitutive update bounds it, 478 -> 474)
+    const int nItems = min(EPB, nEl - (int)blockIdx.x * EPB) * NP;
     if constexpr (sizeof(KT) == 8) {
         // ---- stiffness in FP64, which the FP64 pipe bounds: K_ab = sum_q lt ga(x)gb + mt (gb(x)ga + ga.gb I)
         // - c1 va(x)vb with lt = lam + c2/3, mt = G - c2/2 and lam, G of the element, so that
         //   K = lam A + G (A^T + tr A I) + B/3 - (B^T + tr B I)/2 - V,
         //   A = sum_q ga(x)gb, B = sum_q c2 ga(x)gb, V = sum_q c1 va(x)vb, g with sqrt(|w detJ|) in it and the sign
-        // of w detJ (negative in an inverted element, which the element status reports) given to ga and va:
-        // 9 instructions per pair of nodes and elastic Gauss point, 33 where plastic, against 58 and 88 with the
-        // three terms formed per pair from the split geometry (10,240 hex8 J2 elements, half of them plastic: 659 ->
-        // 326 us with the FP64 pipe 87 % busy before).  The FP64 geometry (not its 48-bit split) is
+        // of w detJ (negative in an inverted element, which the element status reports) given to ga and va, va with
+        // sqrt(|c1|) in it:
+        // 9 instructions per pair of nodes and elastic Gauss point, 30 where plastic, against 58 and 88 with the
+        // three terms formed per pair from the split geometry (10,240 hex8 J2 elements, half of them plastic: 659 us with
+        // the FP64 pipe 87 % busy, 292 now with it 75 to 80 %; 2,500 elements 92).  The FP64 geometry (not its 48-bit split) is
         // scaled once per Gauss point and node, va = n . ga likewise.
         __syncthreads();  // the residual has read g
         if (valid && lane < NQ) {
             const int q = lane;
             const double* gq = geo + ((int64_t)e * NQ + q) * (3 * NN + 1);
             const double sw = sqrt(fabs(gq[3 * NN]));
+            const bool plasticQ = mo.c1 != 0.0 || mo.c2 != 0.0;
+            double n[6];
+            if (plasticQ) {
+                const double rc = sqrt(fabs(mo.c1));
+#pragma unroll
+                for (int i = 0; i < 6; ++i) n[i] = rc * mo.n[i];
+            }
 #pragma unroll 2
             for (int a = 0; a < NN; ++a) {
                 const double g0 = sw * gq[3 * a], g1 = sw * gq[3 * a + 1], g2 = sw * gq[3 * a + 2];
@@ -373,18 +386,19 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
                 gd[0] = g0;
                 gd[1] = g1;
                 gd[2] = g2;
-                if (mo.c1 != 0.0 || mo.c2 != 0.0) {
+                if (plasticQ) {
                     double* vd = &sh.u.d.vd[le][(q * NN + a) * 3];
-                    vd[0] = fma(mo.n[4], g2, fma(mo.n[3], g1, mo.n[0] * g0));
-                    vd[1] = fma(mo.n[5], g2, fma(mo.n[1], g1, mo.n[3] * g0));
-                    vd[2] = fma(mo.n[2], g2, fma(mo.n[5], g1, mo.n[4] * g0));
+                    vd[0] = fma(n[4], g2, fma(n[3], g1, n[0] * g0));
+                    vd[1] = fma(n[5], g2, fma(n[1], g1, n[3] * g0));
+                    vd[2] = fma(n[2], g2, fma(n[5], g1, n[4] * g0));
                 }
             }
         }
         __syncthreads();
-        if (!valid) return;
-        const double lam = pv[6], G = pv[7];
-        for (int p = lane; p < NP; p += TPE) {
+        for (int item = tid; item < nItems; item += SSShared<NN, NQ, KT>::BLOCK) {
+            const int le = item / NP, p = item - le * NP, e = blockIdx.x * EPB + le;
+            const double* pv = propsTable ? propsTable + 8 * (int64_t)elemRow[e] : props.v;
+            const double lam = pv[6], G = pv[7];
             const int a = pair_a(p, NN);
             const int b = a + (p - (a * NN - a * (a - 1) / 2));
             double A[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, B[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -406,8 +420,8 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
                     const double* vA = &sh.u.d.vd[le][(q * NN + a) * 3];
                     const double* vB = &sh.u.d.vd[le][(q * NN + b) * 3];
                     const double cg[3] = {c2 * ga[0], c2 * ga[1], c2 * ga[2]};
-                    const double c1s = flip_sign(c1, neg);
-                    const double cv[3] = {c1s * vA[0], c1s * vA[1], c1s * vA[2]};
+                    const int neg1 = neg ^ (__double2hiint(c1) & 0x80000000);
+                    const double cv[3] = {flip_sign(vA[0], neg1), flip_sign(vA[1], neg1), flip_sign(vA[2], neg1)};
                     const double vb[3] = {vB[0], vB[1], vB[2]};
 #pragma unroll
                     for (int i = 0; i < 3; ++i)
@@ -434,13 +448,13 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
                         k[i][j] += t;
                     }
             }
-            store(p, a, b, k);
+            store(e, p, a, b, k);
         }
         return;
     }
-    if (!valid) return;
     // ---- stiffness: K_ab = sum_q lt ga(x)gb + mt (gb(x)ga + ga.gb I) - c1 va(x)vb ----
-    for (int p = lane; p < NP; p += TPE) {
+    for (int item = tid; item < nItems; item += SSShared<NN, NQ, KT>::BLOCK) {
+        const int le = item / NP, p = item - le * NP;
         const int a = pair_a(p, NN);
         const int b = a + (p - (a * NN - a * (a - 1) / 2));
         KT k[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -474,7 +488,7 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
                     for (int j = 0; j < 3; ++j) k[i][j] -= c1 * va[i] * vb[j];
             }
         }
-        store(p, a, b, k);
+        store(blockIdx.x * EPB + le, p, a, b, k);
     }
 }
 

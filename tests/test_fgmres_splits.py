@@ -58,3 +58,24 @@ def test_fgmres_gram_schmidt_of_every_vector_length(gpu_lib, dims):
     x, y = s.linearSolve(b), s._vec()
     _lib.check(f.lib.ef_bsr_matvec(f.ctx, x.data_ptr(), y.data_ptr(), f._stream()), "ef_bsr_matvec")
     assert float((b - y).norm() / b.norm()) <= 1e-7
+
+
+@pytest.mark.parametrize("dims", [(24, 49, 47), (24, 49, 48)], ids=["60000-nodes", "61250-nodes"])
+def test_fgmres_product_on_both_sides_of_its_streaming_rule(gpu_lib, dims):
+    """The product in the diagonal form reads cached lines up to 60,000 nodes and streams above.  The same check."""
+    from edelweissfe_gb300 import _lib
+    from edelweissfe_gb300.solver import LinSolverOptions, TimeStep
+
+    spec = j2_box_spec(*dims, *[0.1 * k for k in dims])
+    ts = TimeStep(1, 0.1, 0.1, 0.1, 0.1, 0.1)
+    s = build_gpu_solver(spec, linsolver=LinSolverOptions(method="fgmres", rtol=1e-8))
+    f = build_gpu_solver(spec, keFp64=True, linsolver=LinSolverOptions(mixed=False))
+    b = torch.as_tensor(np.random.default_rng(11).normal(size=s.nDof), device="cuda")
+    b[s.dirIdx] = 0.0
+    for g in (s, f):
+        d, P, F = g._vec(), g._vec(), g._vec()
+        g.computeElements(d, d, P, F, ts)
+        g.assembleStiffnessCSR()
+    x, y = s.linearSolve(b), s._vec()
+    _lib.check(f.lib.ef_bsr_matvec(f.ctx, x.data_ptr(), y.data_ptr(), f._stream()), "ef_bsr_matvec")
+    assert float((b - y).norm() / b.norm()) <= 1e-7
