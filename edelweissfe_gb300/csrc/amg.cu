@@ -344,6 +344,38 @@ __global__ void sa_block_copy_kernel(int64_t nP, const int32_t* __restrict__ tId
     if (k < nP) sa_block_copy<BF>(k, tIdx, Pv, dst);
 }
 
+// Loads of matrix values and indices ahead of griddepcontrol.wait: a cycle's small kernels are chains of a few
+// dependent loads (row pointer, index, value, vector), and only the vector comes from the kernel before.  The
+// matrices are set-up results, and the kernel launched just before one of these is always one of the cycle or of the
+// Krylov iteration, so they are complete once the CTA can run.  Volatile, so that they stay ahead of the wait.  us of the
+// cycle before and now: 7,412 nodes of quadratic elements 25.3 -> 23.2, hex8 4,225 nodes 19.3 -> 17.2, 11,849 nodes 27.7 ->
+// 23.5, 18,081 nodes 30.0 -> 25.5, 169,781 nodes 78.1 -> 71.3.
+__device__ __forceinline__ int early(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.nc.s32 %0, [%1];\n" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t early(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];\n" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float early(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];\n" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 early(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 early(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // restriction: a CTA per coarse node, a thread per P block of its column (consecutive blocks of
 // the transpose-order copy), sums in a fixed order (each thread's blocks, a shuffle tree per warp,
 // the warps in order)
@@ -353,12 +385,35 @@ __global__ void __launch_bounds__(kSaRestrictThreads) sa_restrict_onepass_kernel
     int nC, const int32_t* __restrict__ tPtr, const int32_t* __restrict__ rowT,
     const float* __restrict__ PT, const float* __restrict__ t, const uint8_t* __restrict__ coarseDead,
     float* __restrict__ rc) {
-    ef::dep_entry();
     __shared__ float red[kSaRestrictThreads / 32][BC];
     const int I = blockIdx.x;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    // the thread's first block ahead of the wait
+    const int k0 = early(tPtr + I) + (int)threadIdx.x, k1 = early(tPtr + I + 1);
+    float2 P[BF * BC / 2];
+    int m = 0;
+    if (k0 < k1) {
+        m = early(rowT + k0);
+        const float2* src = reinterpret_cast<const float2*>(PT + (int64_t)k0 * BF * BC);
+#pragma unroll
+        for (int i = 0; i < BF * BC / 2; ++i) P[i] = early(src + i);
+    }
+    ef::dep_entry();
     float a[BC];
-    sa_restrict_onepass_partial<BF>(I, threadIdx.x, kSaRestrictThreads, tPtr, rowT, PT, t, a);
+#pragma unroll
+    for (int j = 0; j < BC; ++j) a[j] = 0.f;
+    if (k0 < k1) {
+#pragma unroll
+        for (int i = 0; i < BF; ++i) {
+            const float ti = t[BF * (int64_t)m + i];
+#pragma unroll
+            for (int j = 0; j < BC; j += 2) {
+                a[j] += P[(i * BC + j) / 2].x * ti;
+                a[j + 1] += P[(i * BC + j) / 2].y * ti;
+            }
+        }
+        sa_restrict_onepass_range<BF>(k0 + kSaRestrictThreads, k1, kSaRestrictThreads, rowT, PT, t, a);
+    }
 #pragma unroll
     for (int j = 0; j < BC; ++j) {
 #pragma unroll
@@ -402,26 +457,42 @@ __global__ void __launch_bounds__(kSaRestrictThreads) sa_restrict_onepass_h_kern
     int nC, const int32_t* __restrict__ tPtr, const int32_t* __restrict__ rowT, const uint4* __restrict__ q0,
     const uint4* __restrict__ q1, const uint32_t* __restrict__ q2, const float* __restrict__ t,
     const uint8_t* __restrict__ coarseDead, float* __restrict__ rc) {
-    ef::dep_entry();
     __shared__ float red[kSaRestrictThreads / 32][BC];
     const int I = blockIdx.x;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     float a[BC];
 #pragma unroll
     for (int j = 0; j < BC; ++j) a[j] = 0.f;
-    for (int64_t k = tPtr[I] + threadIdx.x; k < tPtr[I + 1]; k += kSaRestrictThreads) {
-        const uint4 u = q0[k], v = q1[k];
-        const uint32_t w = q2[k];
+    // the thread's first block ahead of the wait
+    int k = early(tPtr + I) + (int)threadIdx.x;
+    const int k1 = early(tPtr + I + 1);
+    uint4 u = {}, v = {};
+    uint32_t w = 0;
+    int m = 0;
+    if (k < k1) {
+        u = early(q0 + k);
+        v = early(q1 + k);
+        w = early(q2 + k);
+        m = early(rowT + k);
+    }
+    ef::dep_entry();
+    while (k < k1) {
         float P[18];
         const uint32_t words[9] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, w};
+        const float t0 = t[3 * (int64_t)m], t1 = t[3 * (int64_t)m + 1], t2 = t[3 * (int64_t)m + 2];
+        k += kSaRestrictThreads;
+        if (k < k1) {
+            u = q0[k];
+            v = q1[k];
+            w = q2[k];
+            m = rowT[k];
+        }
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
             const float2 f = sa_unpack_bf16x2(words[q]);
             P[2 * q] = f.x;
             P[2 * q + 1] = f.y;
         }
-        const int64_t m = rowT[k];
-        const float t0 = t[3 * m], t1 = t[3 * m + 1], t2 = t[3 * m + 2];
 #pragma unroll
         for (int j = 0; j < BC; ++j) a[j] += P[j] * t0 + P[BC + j] * t1 + P[2 * BC + j] * t2;
     }
@@ -681,53 +752,65 @@ __device__ __forceinline__ float2 ldv2(const float* p) {
     return *reinterpret_cast<const float2*>(p);
 }
 // H: the block values come from a BF16 copy (valsH, 6 values = three 4-byte words per block row)
-// the sum over blocks first, first + step, ... (15 at a time) of a row
+// three blocks k0, k0 + 5, k0 + 10 of a lane (15 per warp), their loads issued together; c < 0: none
+template <bool H, bool EARLY>
+__device__ __forceinline__ void resid6_load(int k0, int e, int ri, const int32_t* __restrict__ colIdx,
+                                            const float* __restrict__ vals, const uint32_t* __restrict__ valsH, int (&c)[3],
+                                            float2 (&a)[3][3]) {
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+        const int k = k0 + 5 * u;
+        c[u] = -1;
+        if (k < e) {
+            c[u] = BC * (EARLY ? early(colIdx + k) : colIdx[k]);
+            if (H) {
+                const uint32_t* v = valsH + ((int64_t)k * BC * BC + BC * ri) / 2;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const uint32_t w = EARLY ? early(v + q) : v[q];
+                    a[u][q] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+                }
+            } else {
+                const float2* v = reinterpret_cast<const float2*>(vals + (int64_t)k * BC * BC + BC * ri);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) a[u][q] = EARLY ? early(v + q) : v[q];
+            }
+        }
+    }
+}
+template <bool CG>
+__device__ __forceinline__ void resid6_add(const int (&c)[3], const float2 (&a)[3][3], const float* x, float& acc) {
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+        if (c[u] >= 0) {
+            const float2 x0 = ldv2<CG>(x + c[u]), x1 = ldv2<CG>(x + c[u] + 2), x2 = ldv2<CG>(x + c[u] + 4);
+            acc += a[u][0].x * x0.x + a[u][0].y * x0.y + a[u][1].x * x1.x + a[u][1].y * x1.y + a[u][2].x * x2.x +
+                   a[u][2].y * x2.y;
+        }
+}
+__device__ __forceinline__ float resid6_lanes(float acc) {
+    // lanes i < 6: acc(i) + acc(i + 6) + acc(i + 12) + acc(i + 18) + acc(i + 24)
+    const float s1 = acc + __shfl_down_sync(0xffffffffu, acc, 6);
+    const float s2 = s1 + __shfl_down_sync(0xffffffffu, s1, 12);
+    return s2 + __shfl_down_sync(0xffffffffu, acc, 24);
+}
+// the sum over the blocks of a row, 15 at a time
 template <bool CG, bool H = false>
-__device__ __forceinline__ float resid6_sum(int m, int lane, int first, int step, const int32_t* __restrict__ rowPtr,
+__device__ __forceinline__ float resid6_sum(int m, int lane, const int32_t* __restrict__ rowPtr,
                                             const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
                                             const float* x, const uint32_t* __restrict__ valsH) {
     const int g = lane / BC, ri = lane - BC * g;
     float acc = 0.f;
     if (g < 5) {
-        // three blocks per lane and step (15 per warp), their loads issued together
         const int e = rowPtr[m + 1];
-        for (int k0 = rowPtr[m] + first + g; k0 < e; k0 += step) {
+        for (int k0 = rowPtr[m] + g; k0 < e; k0 += 15) {
             int c[3];
             float2 a[3][3];
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                const int k = k0 + 5 * u;
-                c[u] = -1;
-                if (k < e) {
-                    c[u] = BC * colIdx[k];
-                    if (H) {
-                        const uint32_t* v = valsH + ((int64_t)k * BC * BC + BC * ri) / 2;
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            const uint32_t w = v[q];
-                            a[u][q] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
-                        }
-                    } else {
-                        const float2* v = reinterpret_cast<const float2*>(vals + (int64_t)k * BC * BC + BC * ri);
-                        a[u][0] = v[0];
-                        a[u][1] = v[1];
-                        a[u][2] = v[2];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                if (c[u] >= 0) {
-                    const float2 x0 = ldv2<CG>(x + c[u]), x1 = ldv2<CG>(x + c[u] + 2), x2 = ldv2<CG>(x + c[u] + 4);
-                    acc += a[u][0].x * x0.x + a[u][0].y * x0.y + a[u][1].x * x1.x + a[u][1].y * x1.y +
-                           a[u][2].x * x2.x + a[u][2].y * x2.y;
-                }
+            resid6_load<H, false>(k0, e, ri, colIdx, vals, valsH, c, a);
+            resid6_add<CG>(c, a, x, acc);
         }
     }
-    // lanes i < 6: acc(i) + acc(i + 6) + acc(i + 12) + acc(i + 18) + acc(i + 24)
-    const float s1 = acc + __shfl_down_sync(0xffffffffu, acc, 6);
-    const float s2 = s1 + __shfl_down_sync(0xffffffffu, s1, 12);
-    return s2 + __shfl_down_sync(0xffffffffu, acc, 24);
+    return resid6_lanes(acc);
 }
 
 // the row's end: component i of the product, yi, in lane i < 6 of the warp
@@ -754,7 +837,7 @@ __device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __res
                                            const float* x, const float* r, const uint8_t* __restrict__ mask, float* t,
                                            const float* __restrict__ binv, float omega,
                                            const uint32_t* __restrict__ valsH = nullptr, float ys = 1.f) {
-    const float yi = resid6_sum<CG, H>(m, lane, 0, 15, rowPtr, colIdx, vals, x, valsH);
+    const float yi = resid6_sum<CG, H>(m, lane, rowPtr, colIdx, vals, x, valsH);
     resid6_end<CG>(m, lane, yi, x, r, mask, t, binv, omega, ys);
 }
 
@@ -778,16 +861,34 @@ __global__ void __launch_bounds__(256) level_residual6_kernel(int nN, const int3
 // The same with W warps per row, for levels of too few rows to fill the GPU with a warp each (the row is then a
 // chain of dependent loads, 15 blocks at a time): warp w takes blocks 15 w, 15 (w + W), ... and warp 0
 // adds the warps' sums in order
-template <int W>
+template <int W, bool H>
 __global__ void __launch_bounds__(32 * W) level_residual6_split_kernel(
     int nN, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ colIdx, const float* __restrict__ vals,
     const float* __restrict__ x, const float* __restrict__ r, const uint8_t* __restrict__ mask, float* __restrict__ t,
     const float* __restrict__ binv, float omega, const uint32_t* __restrict__ valsH, float ys) {
-    ef::dep_entry();
     __shared__ float part[W][BC];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = blockIdx.x;
-    float yi = valsH ? resid6_sum<false, true>(m, lane, 15 * w, 15 * W, rowPtr, colIdx, vals, x, valsH)
-                     : resid6_sum<false, false>(m, lane, 15 * w, 15 * W, rowPtr, colIdx, vals, x, nullptr);
+    const int g = lane / BC, ri = lane - BC * g;
+    // the warp's first blocks ahead of the wait
+    const int e = early(rowPtr + m + 1);
+    int k0 = early(rowPtr + m) + 15 * w + g, c[3] = {-1, -1, -1};
+    float2 a[3][3];
+    if (g < 5) {
+        if (H)
+            resid6_load<true, true>(k0, e, ri, colIdx, vals, valsH, c, a);
+        else
+            resid6_load<false, true>(k0, e, ri, colIdx, vals, valsH, c, a);
+    }
+    ef::dep_entry();
+    float acc = 0.f;
+    if (g < 5) {
+        resid6_add<false>(c, a, x, acc);
+        for (k0 += 15 * W; k0 < e; k0 += 15 * W) {
+            resid6_load<H, false>(k0, e, ri, colIdx, vals, valsH, c, a);
+            resid6_add<false>(c, a, x, acc);
+        }
+    }
+    float yi = resid6_lanes(acc);
     if (lane < BC) part[w][lane] = yi;
     __syncthreads();
     if (w != 0) return;
@@ -850,19 +951,44 @@ __global__ void __launch_bounds__(W == 1 ? 256 : 32 * W) sa_post6_fused_kernel(
     int nN, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ col, const float* __restrict__ C,
     const float* __restrict__ e, const float* __restrict__ r, const float* __restrict__ t,
     const float* __restrict__ binv, const uint8_t* __restrict__ dead, float omega, float* __restrict__ x) {
-    ef::dep_entry();
     const int lane = threadIdx.x & 31, w = W == 1 ? 0 : threadIdx.x >> 5;
     const int m = W == 1 ? (blockIdx.x * blockDim.x + threadIdx.x) >> 5 : blockIdx.x;
-    if (m >= nN) return;  // whole warps
     const int k0 = lane / BC, i = lane % BC;
-    float y = 0.f;
-    if (k0 < 5)
-        for (int a = rowPtr[m] + 5 * w + k0; a < rowPtr[m + 1]; a += 5 * W) {
-            const float* cr = C + (int64_t)a * BC * BC + i * BC;
-            const float* ev = e + BC * (int64_t)col[a];
+    // the warp's first blocks and the block inverse's row ahead of the wait
+    int a = 0, a1 = 0, c0 = 0;
+    float2 cf[BC / 2], Bf[BC / 2];
+    if (m < nN) {
+        a = early(rowPtr + m) + 5 * w + k0;
+        a1 = k0 < 5 ? early(rowPtr + m + 1) : 0;
+        if (a < a1) {
+            c0 = early(col + a);
+            const float2* cr = reinterpret_cast<const float2*>(C + (int64_t)a * BC * BC + i * BC);
 #pragma unroll
-            for (int j = 0; j < BC; ++j) y += cr[j] * ev[j];
+            for (int j = 0; j < BC / 2; ++j) cf[j] = early(cr + j);
         }
+        if (w == 0 && lane < BC) {
+            const float2* B = reinterpret_cast<const float2*>(binv + (int64_t)m * BC * BC + i * BC);
+#pragma unroll
+            for (int j = 0; j < BC / 2; ++j) Bf[j] = early(B + j);
+        }
+    }
+    ef::dep_entry();
+    if (m >= nN) return;  // whole warps
+    float y = 0.f;
+    if (a < a1) {
+        const float* ev = e + BC * (int64_t)c0;
+#pragma unroll
+        for (int j = 0; j < BC / 2; ++j) {
+            y += cf[j].x * ev[2 * j];
+            y += cf[j].y * ev[2 * j + 1];
+        }
+    }
+    for (a += 5 * W; a < a1; a += 5 * W) {
+        const float* cr = C + (int64_t)a * BC * BC + i * BC;
+        const float* ev = e + BC * (int64_t)col[a];
+#pragma unroll
+        for (int j = 0; j < BC; ++j) y += cr[j] * ev[j];
+    }
     // lane i gathers lanes i + 6, i + 12, i + 18, i + 24 in that order
     float s = y;
 #pragma unroll
@@ -880,10 +1006,10 @@ __global__ void __launch_bounds__(W == 1 ? 256 : 32 * W) sa_post6_fused_kernel(
             for (int q = 1; q < W; ++q) s += part[q][lane];
     }
     if (lane < BC) {
-        const float* B = binv + (int64_t)m * BC * BC + i * BC;
         float z = 0.f;
 #pragma unroll
-        for (int q = 0; q < BC; ++q) z += B[q] * (r[BC * (int64_t)m + q] + t[BC * (int64_t)m + q]);
+        for (int q = 0; q < BC; ++q)
+            z += (q & 1 ? Bf[q / 2].y : Bf[q / 2].x) * (r[BC * (int64_t)m + q] + t[BC * (int64_t)m + q]);
         x[BC * (int64_t)m + i] = dead[BC * (int64_t)m + i] ? 0.f : omega * z + s;
     }
 }
@@ -1083,21 +1209,34 @@ __global__ void coarsest_inverse_kernel(int nN, const int32_t* __restrict__ rowP
 // x = inv r on the coarsest level (dead DOFs -> 0), one warp per row (coalesced row of inv,
 // fixed shuffle tree)
 template <bool CG>
-__device__ __forceinline__ void coarsest_row(int i, int lane, int n, const float* __restrict__ inv, const float* r,
-                                             const uint8_t* __restrict__ dead, float* x) {
-    float s = 0.f;
-    for (int j = lane; j < n; j += 32) s += inv[(int64_t)i * n + j] * ldv<CG>(r + j);
+__device__ __forceinline__ void coarsest_end(int i, int lane, float s, const uint8_t* __restrict__ dead, float* x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) stv<CG>(x + i, dead[i] ? 0.f : s);
 }
+template <bool CG>
+__device__ __forceinline__ void coarsest_row(int i, int lane, int n, const float* __restrict__ inv, const float* r,
+                                             const uint8_t* __restrict__ dead, float* x) {
+    float s = 0.f;
+    for (int j = lane; j < n; j += 32) s += inv[(int64_t)i * n + j] * ldv<CG>(r + j);
+    coarsest_end<CG>(i, lane, s, dead, x);
+}
 
 __global__ void coarsest_apply_kernel(int n, const float* __restrict__ inv, const float* __restrict__ r,
                                       const uint8_t* __restrict__ dead, float* __restrict__ x) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    constexpr int kAhead = 8;  // values of a lane loaded ahead of the wait
+    float v[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) v[q] = i < n && lane + 32 * q < n ? early(inv + (int64_t)i * n + lane + 32 * q) : 0.f;
     ef::dep_entry();
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= n) return;
-    coarsest_row<false>(i, threadIdx.x & 31, n, inv, r, dead, x);
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+        if (lane + 32 * q < n) s += v[q] * r[lane + 32 * q];
+    for (int j = lane + 32 * kAhead; j < n; j += 32) s += inv[(int64_t)i * n + j] * r[j];
+    coarsest_end<false>(i, lane, s, dead, x);
 }
 
 // The multigrid cycle below a level as one launch: one cluster of kCoarseCtas CTAs runs the
@@ -1454,7 +1593,8 @@ ef_status ef_launch_level_residual(int bs, int nN, const int32_t* rowPtr, const 
                 x, r, mask, t, binv, omega));
     } else {
         if (row_warps(nN) > 1)
-            EF_CUDA(ef::launch_dep(level_residual6_split_kernel<kRowWarps>, nN, 32 * kRowWarps, 0, s, nN, rowPtr, colIdx,
+            EF_CUDA(ef::launch_dep(valsH ? level_residual6_split_kernel<kRowWarps, true>
+                                         : level_residual6_split_kernel<kRowWarps, false>, nN, 32 * kRowWarps, 0, s, nN, rowPtr, colIdx,
                                    vals, x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
         else
             EF_CUDA(ef::launch_dep(level_residual6_kernel, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, colIdx, vals,

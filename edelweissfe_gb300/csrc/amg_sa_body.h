@@ -455,14 +455,11 @@ EF_SA_HD void sa_block_copy(int64_t k, const int32_t* __restrict__ tIdx, const f
 }
 
 // restriction, one thread's share of coarse node I from the transpose-order copy PT:
-// a[j] = sum over k = tPtr[I] + lane, + nLanes, ... of sum_i PT_k[i][j] t[rowT[k]][i]
+// a[j] += sum over k = k0, k0 + nLanes, ... < k1 of sum_i PT_k[i][j] t[rowT[k]][i]
 template <int BF>
-EF_SA_HD void sa_restrict_onepass_partial(int I, int lane, int nLanes, const int32_t* __restrict__ tPtr,
-                                          const int32_t* __restrict__ rowT, const float* __restrict__ PT,
-                                          const float* __restrict__ t, float a[BC]) {
-    EF_SA_UNROLL
-    for (int j = 0; j < BC; ++j) a[j] = 0.f;
-    for (int64_t k = tPtr[I] + lane; k < tPtr[I + 1]; k += nLanes) {
+EF_SA_HD void sa_restrict_onepass_range(int64_t k0, int64_t k1, int nLanes, const int32_t* __restrict__ rowT,
+                                        const float* __restrict__ PT, const float* __restrict__ t, float a[BC]) {
+    for (int64_t k = k0; k < k1; k += nLanes) {
         float P[BF * BC];
         sa_load_block<BF>(PT + k * BF * BC, P);
         const int64_t m = rowT[k];
@@ -474,6 +471,15 @@ EF_SA_HD void sa_restrict_onepass_partial(int I, int lane, int nLanes, const int
             EF_SA_UNROLL
             for (int j = 0; j < BC; ++j) a[j] += P[i * BC + j] * ti[i];
     }
+}
+// the share of lane of column I of P: a[j] = sum over k = tPtr[I] + lane, + nLanes, ...
+template <int BF>
+EF_SA_HD void sa_restrict_onepass_partial(int I, int lane, int nLanes, const int32_t* __restrict__ tPtr,
+                                          const int32_t* __restrict__ rowT, const float* __restrict__ PT,
+                                          const float* __restrict__ t, float a[BC]) {
+    EF_SA_UNROLL
+    for (int j = 0; j < BC; ++j) a[j] = 0.f;
+    sa_restrict_onepass_range<BF>(tPtr[I] + lane, tPtr[I + 1], nLanes, rowT, PT, t, a);
 }
 
 // prolongation product of block b (row order): q[i] = sum_j P_b[i][j] xc[col(b)][j]
