@@ -20,13 +20,15 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "amg_sa_body.h"
+#include "early.cuh"
 #include "ef_common.cuh"
 
 namespace ef {
 
 constexpr int kSellThreads = 128;  // four warps per CTA
-constexpr int kSellSlicesPerCta = kSellThreads / 32;  // the product: a warp per slice
 // Split slices: S warps per slice, each taking a contiguous share of the slice's entries, four
 // warps per CTA up to S = 4 and S warps (one slice) above
 
@@ -199,6 +201,10 @@ __device__ __forceinline__ void sell_block_add(const float (&a)[9], const float 
 // by bulk copies was slower (preconditioner 100 us), as fewer warps gather.
 constexpr int kSellBatch = 2;
 
+// The first two columns are loaded ahead of the wait for the kernel before (early.cuh), which gives a product of
+// 785 nodes of quadratic elements 8.2 -> 7.4 us, of 7,412 nodes 10.4 -> 9.7, of 19,456 nodes of a tied mesh 13.8 -> 12.6.  The
+// same in the diagonal form gains nothing, and in the residual and the post-smoothing it costs the large
+// systems more (cycle at 169,781 nodes 71.2 -> 74.3 and 72.4 us) than it gives the small.
 // y = sc K x on the free DOFs (0 on masked rows); COPY: xcopy = sc x as well; sc = *scale (1 without
 // one: the FGMRES basis vector x then carries its normalisation factor); S warps per slice
 template <bool COPY, int S>
@@ -207,29 +213,40 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
     const int32_t* __restrict__ col, const float* __restrict__ v9, const float* __restrict__ x,
     const uint8_t* __restrict__ mask, float* __restrict__ y, float* __restrict__ xcopy,
     const float* __restrict__ scale, const float* __restrict__ binv) {
-    ef::dep_entry();
     SellPart p;
     const bool active = sell_part<S>(nSlices, off, p);
     float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-    if (active) {
-        const int32_t* cs = col + p.e0 + p.lane;
-        const float* vs = v9 + 9 * p.e0 + p.lane;
-        for (int j = p.j0; j < p.j1; j += kSellBatch) {
-            float a[kSellBatch][9], xv[kSellBatch][3];
+    float a[kSellBatch][9];
+    int c3[kSellBatch];
+    const int32_t* cs = col + p.e0 + p.lane;
+    const float* vs = v9 + 9 * p.e0 + p.lane;
+    auto load = [&](int j, auto ahead) {
 #pragma unroll
-            for (int u = 0; u < kSellBatch; ++u) {
-                const int k = min(j + u, p.j1 - 1);
-                const int c3 = 3 * __ldcs(cs + 32 * k);
+        for (int u = 0; u < kSellBatch; ++u) {
+            const int k = min(j + u, p.j1 - 1);
+            c3[u] = 3 * (ahead() ? early_cs(cs + 32 * k) : __ldcs(cs + 32 * k));
 #pragma unroll
-                for (int i = 0; i < 9; ++i) a[u][i] = __ldcs(vs + 288 * k + 32 * i);
+            for (int i = 0; i < 9; ++i)
+                a[u][i] = ahead() ? early_cs(vs + 288 * k + 32 * i) : __ldcs(vs + 288 * k + 32 * i);
+        }
+    };
+    const bool some = active && p.j0 < p.j1;
+    if (some) load(p.j0, std::true_type());
+    ef::dep_entry();
+    if (some)
+        for (int j = p.j0;;) {
+            float xv[kSellBatch][3];
 #pragma unroll
-                for (int i = 0; i < 3; ++i) xv[u][i] = x[c3 + i];
-            }
+            for (int u = 0; u < kSellBatch; ++u)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) xv[u][i] = x[c3[u] + i];
 #pragma unroll
             for (int u = 0; u < kSellBatch; ++u)
                 if (j + u < p.j1) sell_block_add(a[u], xv[u], y0, y1, y2);
+            j += kSellBatch;
+            if (j >= p.j1) break;
+            load(j, std::false_type());
         }
-    }
     if (!sell_combine<S>(p, active, y0, y1, y2)) return;
     const int r = p.sl * 32 + p.lane;
     if (r >= nN) return;
@@ -507,9 +524,6 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sa_post_fused_kernel(
 
 using namespace ef;
 
-static inline unsigned sell_grid(int nSlices) {
-    return (unsigned)((nSlices + kSellSlicesPerCta - 1) / kSellSlicesPerCta);
-}
 static inline unsigned sell_split_grid(int nSlices, int S) {
     const int spc = sell_split_threads(S) / (32 * S);
     return (unsigned)((nSlices + spc - 1) / spc);
