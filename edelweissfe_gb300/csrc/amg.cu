@@ -125,16 +125,44 @@ __global__ void sa_prolongator_kernel(int64_t nP, const int32_t* __restrict__ pR
     sa_prolongator_block<BF>(b, pRow, pCol, pSeg, pSrc, fineCol, fineVals, fineMask, offs, agg, binv, *wP, Pv);
 }
 
-// one AP block per thread
+// A thread per pair of values of an AP block (row i, columns j and j + 1), which adds the block's pairs in list order: the sums
+// of sa_ap_block.  The threads of a block read the same indices and matrix rows and neighbouring values of P.  With a
+// thread per block the few blocks of the coarse levels were long serial chains: fine and first coarse level of a tied mesh
+// of 19,456 nodes 492 -> 200 and 489 -> 43 us, of 7,412 nodes of quadratic elements 233 -> 92 us.  Where the pair
+// products of a group of rows fit the shared memory, sa_ap_rows_kernel is faster (169,781 nodes 581 against 710 us, its
+// first coarse level 36 against 48).
 template <int BF>
-__global__ void sa_ap_kernel(int64_t nAP, const int32_t* __restrict__ apRow, const int64_t* __restrict__ apSeg,
-                             const int32_t* __restrict__ apK, const int32_t* __restrict__ apP,
-                             const int32_t* __restrict__ fineCol, const float* __restrict__ fineVals,
-                             const uint8_t* __restrict__ fineMask, const float* __restrict__ Pv,
-                             float* __restrict__ APv) {
-    const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) sa_ap_kernel(int64_t nAP, const int32_t* __restrict__ apRow,
+                                                    const int64_t* __restrict__ apSeg, const int32_t* __restrict__ apK,
+                                                    const int32_t* __restrict__ apP, const int32_t* __restrict__ fineCol,
+                                                    const float* __restrict__ fineVals,
+                                                    const uint8_t* __restrict__ fineMask, const float* __restrict__ Pv,
+                                                    float* __restrict__ APv) {
+    constexpr int T = BF * BC / 2;
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t a = idx / T;
     if (a >= nAP) return;
-    sa_ap_block<BF>(a, apRow, apSeg, apK, apP, fineCol, fineVals, fineMask, Pv, APv);
+    const int p = (int)(idx - a * T), i = p / (BC / 2), j2 = p - i * (BC / 2);
+    float2 acc = make_float2(0.f, 0.f);
+    if (!fineMask || !fineMask[BF * (int64_t)apRow[a] + i]) {
+        const int64_t t1 = apSeg[a + 1];
+#pragma unroll 2
+        for (int64_t t = apSeg[a]; t < t1; ++t) {
+            const int32_t k = apK[t];
+            const int64_t n = fineCol[k];
+            const float* v = fineVals + (int64_t)k * BF * BF + i * BF;
+            const float2* P = reinterpret_cast<const float2*>(Pv + (int64_t)apP[t] * BF * BC) + j2;
+#pragma unroll
+            for (int q = 0; q < BF; ++q) {
+                const float av = v[q];
+                const float2 pv = P[q * (BC / 2)];
+                if (fineMask && fineMask[BF * n + q]) continue;
+                acc.x += av * pv.x;
+                acc.y += av * pv.y;
+            }
+        }
+    }
+    reinterpret_cast<float2*>(APv)[idx] = acc;
 }
 
 // AP by groups of kSaApRows finer rows: a thread per pair (coalesced pair lists) leaves the pair's
@@ -810,6 +838,7 @@ __device__ __forceinline__ void resid6_row(int m, int lane, const int32_t* __res
     resid6_end<CG>(m, lane, yi, x, r, mask, t, binv, omega, ys);
 }
 
+template <bool H>
 __global__ void __launch_bounds__(256) level_residual6_kernel(int nN, const int32_t* __restrict__ rowPtr,
                                                                const int32_t* __restrict__ colIdx,
                                                                const float* __restrict__ vals,
@@ -817,14 +846,27 @@ __global__ void __launch_bounds__(256) level_residual6_kernel(int nN, const int3
                                                                const uint8_t* __restrict__ mask, float* __restrict__ t,
                                                                const float* __restrict__ binv, float omega,
                                                                const uint32_t* __restrict__ valsH, float ys) {
-    ef::dep_entry();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, g = lane / BC, ri = lane - BC * g;
     const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // the row's first blocks ahead of the wait
+    int e = 0, k0 = 0, c[3] = {-1, -1, -1};
+    float2 a[3][3];
+    if (m < nN && g < 5) {
+        e = early(rowPtr + m + 1);
+        k0 = early(rowPtr + m) + g;
+        resid6_load<H, true>(k0, e, ri, colIdx, vals, valsH, c, a);
+    }
+    ef::dep_entry();
     if (m >= nN) return;
-    if (valsH)
-        resid6_row<false, true>(m, lane, rowPtr, colIdx, vals, x, r, mask, t, binv, omega, valsH, ys);
-    else
-        resid6_row<false, false>(m, lane, rowPtr, colIdx, vals, x, r, mask, t, binv, omega, nullptr, ys);
+    float acc = 0.f;
+    if (g < 5) {
+        resid6_add<false>(c, a, x, acc);
+        for (k0 += 15; k0 < e; k0 += 15) {
+            resid6_load<H, false>(k0, e, ri, colIdx, vals, valsH, c, a);
+            resid6_add<false>(c, a, x, acc);
+        }
+    }
+    resid6_end<false>(m, lane, resid6_lanes(acc), x, r, mask, t, binv, omega, ys);
 }
 
 // The same with W warps per row, for levels of too few rows to fill the GPU with a warp each (the row is then a
@@ -1566,7 +1608,7 @@ ef_status ef_launch_level_residual(int bs, int nN, const int32_t* rowPtr, const 
                                          : level_residual6_split_kernel<kRowWarps, false>, nN, 32 * kRowWarps, 0, s, nN, rowPtr, colIdx,
                                    vals, x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
         else
-            EF_CUDA(ef::launch_dep(level_residual6_kernel, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, colIdx, vals,
+            EF_CUDA(ef::launch_dep(valsH ? level_residual6_kernel<true> : level_residual6_kernel<false>, nb_((int64_t)nN * 32, 256), 256, 0, s, nN, rowPtr, colIdx, vals,
                                    x, r, mask, t, binv, omega, (const uint32_t*)valsH, ys));
     }
     EF_CUDA(cudaGetLastError());
@@ -1628,7 +1670,7 @@ ef_status ef_launch_sa_setup(int bf, int64_t nP, const int32_t* pRow, const int3
                                  ef::counted(s)>>>(nF, apCap, apRowPtr, apSeg, apK, apP, fineCol, fineVals,    \
                                                    fineMask, Pv, APv);                                         \
     else                                                                                                       \
-        sa_ap_kernel<BF_><<<nb_(nAP, 128), 128, 0, ef::counted(s)>>>(nAP, apRow, apSeg, apK, apP, fineCol,    \
+        sa_ap_kernel<BF_><<<nb_(nAP * (BF_ * BC / 2), 256), 256, 0, ef::counted(s)>>>(nAP, apRow, apSeg, apK, apP, fineCol,    \
                                                                     fineVals, fineMask, Pv, APv);             \
     if (galWarp)                                                                                               \
         sa_galerkin_warp_kernel<BF_><<<nb_(nC, kGalWarps), 32 * kGalWarps, 0, ef::counted(s)>>>(               \
