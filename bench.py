@@ -41,10 +41,10 @@ PROPS = [210000.0, 0.3, 250.0, 1000.0, 0.0, 0.0]
 METRIC = "hex8 J2 load-step s: learned-FGMRES vs Jacobi-PCG @1e-8 resid; assembly GB/s"
 # DRAM bytes (read + write) per launch of the fine-level kernels of the FGMRES solve on the
 # 100x40x40 box (509,343 DOF, 4,406,941 blocks; the slices in their diagonal form), from one ncu
-# capture of bench.py --profile --method fgmres
-SWEEP_TRAFFIC_BYTES = 87.45e6
-PRODUCT_TRAFFIC_BYTES = 176.73e6  # each slice split over 4 warps (170.52e6 with one warp per slice)
-POST_TRAFFIC_BYTES = 95.23e6
+# capture of a load increment
+SWEEP_TRAFFIC_BYTES = 85.19e6
+PRODUCT_TRAFFIC_BYTES = 88.75e6  # half the blocks (176.73e6 from all of them)
+POST_TRAFFIC_BYTES = 93.19e6
 # Newton iterations of the timed increment (13) of the 100x40x40 model: the same in the all-FP64
 # and the mixed-precision GPU solves; the CPU arms charge this many element passes and solves
 PCG_NEWTON_PER_STEP = 8
@@ -512,12 +512,12 @@ def run_ours(a):
 
         # the dominant kernel of the load step: the FGMRES product (one launch per iteration, the
         # largest); the fused post-smoothing and the fine residual (one launch each per iteration) beside
-        roofline = entry(1, "sell_spmv3_kernel (FGMRES product K z, FP32 sliced-ELL in its diagonal form: "
-                            "columns computed from 27 node offsets; one launch per iteration)",
+        roofline = entry(1, "sell_spmv3_dia_kernel (FGMRES product K z, FP32 diagonals of half the matrix, the "
+                            "blocks below read as transposes; one launch per iteration)",
                          PRODUCT_TRAFFIC_BYTES)
         roofline.update({"bound": "hbm", "peak": peaks["hbm_gbs"], "peak_kind": peak_kind, "unit": "GB/s",
-                         "traffic_source": "ncu (dram__bytes_read.sum + dram__bytes_write.sum per launch) of "
-                                           "bench.py --profile --method fgmres",
+                         "traffic_source": "ncu (dram__bytes_read.sum + dram__bytes_write.sum per launch) of a load "
+                                           "increment of this box",
                          "timing": "CUDA events, 50 back-to-back launches on the timed increment's last system"})
         if sp_n and sp_ms > 0:
             # the product's own launches inside the solve: CUDA events around each one on the solve's
