@@ -1859,7 +1859,8 @@ ef_status ef_launch_coarsest_inverse(int nN, const int32_t* rowPtr, const int32_
         return EF_ERR_ARG;
     }
     const size_t smem = sizeof(float) * BC * nN * (2 * BC * nN + 1);
-    EF_CUDA(cudaFuncSetAttribute(coarsest_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    size_t room = 0;  // (96 unknowns take 74 KB)
+    EF_CUDA(ef::smem_room((const void*)coarsest_inverse_kernel, &room));
     coarsest_inverse_kernel<<<1, dim3(32, 32), smem, ef::counted(s)>>>(nN, rowPtr, colIdx, vals, inv);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
@@ -1942,12 +1943,8 @@ ef_status ef_launch_level_residual_bf16_staged(int nSM, int cap, int nN, int64_t
     const uint4* v8 = (const uint4*)vals;
     const __nv_bfloat16* v1 = (const __nv_bfloat16*)(v8 + nBlocks);
     const size_t smem = 2 * ((stage_bytes_bf16(cap) + 15) & ~(size_t)15);
-    static size_t attrSet = 0;
-    if (smem > 48 * 1024 && smem > attrSet) {
-        EF_CUDA(cudaFuncSetAttribute(level_residual3_bf16_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-        attrSet = smem;
-    }
+    size_t room = 0;
+    EF_CUDA(ef::smem_room((const void*)level_residual3_bf16_staged_kernel, &room));
     int perSM = 0;
     EF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, level_residual3_bf16_staged_kernel, kStageThreads,
                                                           smem));

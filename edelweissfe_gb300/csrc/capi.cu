@@ -3,6 +3,10 @@
 // results.  The system, solver, multigrid, learned-correction and batch entry points are in
 // system.cu, solve.cu, precond.cu, learned_api.cu and batch_api.cu.
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "ctx.h"
 
 // launch counter (see ef_common.cuh); launches issued during a stream capture are credited to the
@@ -27,6 +31,27 @@ bool ef::dep_launch_enabled() {
     return on;
 }
 
+cudaError_t ef::smem_room(const void* kernel, size_t* room) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, const void*>, size_t> known;
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto it = known.find({dev, kernel});
+    if (it != known.end()) {
+        *room = it->second;
+        return cudaSuccess;
+    }
+    cudaFuncAttributes fa;
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    const int dynamic = std::max(0, most - (int)fa.sharedSizeBytes);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic);
+    if (e == cudaSuccess) *room = known[{dev, kernel}] = (size_t)dynamic;
+    return e;
+}
 
 static thread_local std::string g_err;
 void ef_set_error(const std::string& s) { g_err = s; }

@@ -56,6 +56,12 @@ inline cudaError_t launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The dynamic shared memory that a launch of `kernel` may ask for on the current device, in *room: all that the device
+// gives less the kernel's static part, allowed once per kernel and device.  The limit is an attribute of the function,
+// which every context and host thread shares, so nobody sets it to what a system of its own needs: a smaller
+// system's would take effect between a larger one's and its launch, which then fails.
+cudaError_t smem_room(const void* kernel, size_t* room);
+
 enum MatKind { MAT_LINEAR_ELASTIC = 0, MAT_VON_MISES = 1, MAT_NEOHOOKE_WA = 2 };
 
 // Constant tables of one element type (shape-function derivatives at the B/J

@@ -693,11 +693,8 @@ ef_status ef_launch_spmv_f32_staged(int nSM, int cap, int nN, const int32_t* row
                                     const float* vals, const float* x, const uint8_t* mask, float* y, float* xcopy,
                                     cudaStream_t s) {
     const size_t smem = 2 * ((sp_stage_bytes(cap) + 15) & ~(size_t)15);
-    static size_t attrSet = 0;
-    if (smem > 48 * 1024 && smem > attrSet) {
-        EF_CUDA(cudaFuncSetAttribute(spmv_f32_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attrSet = smem;
-    }
+    size_t room = 0;
+    EF_CUDA(ef::smem_room((const void*)spmv_f32_staged_kernel, &room));
     int perSM = 0;
     EF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, spmv_f32_staged_kernel, kFB, smem));
     if (perSM < 1) {

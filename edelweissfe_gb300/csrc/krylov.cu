@@ -856,14 +856,11 @@ static bool plan_for(int vDouble, const PcgShape& shape, int nNodes, const int32
     const size_t vt = vDouble ? sizeof(double) : sizeof(float);
     const int grid = shape.grid, lpr = shape.lpr;
     const int per = (nNodes + grid - 1) / grid, rpw = 32 / lpr, groups = (per + rpw - 1) / rpw;
-    int dev = 0, most = 0;
-    cudaFuncAttributes fa;
-    const void* kernel = pcg_resident(vDouble, lpr, shape.cluster);
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, kernel) != cudaSuccess)
+    size_t room = 0;
+    if (ef::smem_room(pcg_resident(vDouble, lpr, shape.cluster), &room) != cudaSuccess) {
+        (void)cudaGetLastError();
         return false;
-    const size_t room = (size_t)std::max(0, most - (int)fa.sharedSizeBytes);
+    }
     p = PcgResidentPlan();
     p.shape = shape;
     // the steps first: they need no halo, so that a large system's plan is not begun
@@ -925,12 +922,6 @@ static cudaLaunchConfig_t cluster_config(const PcgShape& shape, int vDouble, siz
     return cfg;
 }
 
-static cudaError_t resident_attributes(const void* k, bool cluster, size_t smem) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return e;
-}
-
 // The rule of the dispatch.  A system that fits into one cluster's shared memory (about 3,200 rows of 27
 // blocks in FP32, 1,600 in FP64) runs there: a reduction through the cluster's barrier costs about a third
 // of one through L2.  Else one that fits into all SMs' shared memory runs in the grid form.  Else
@@ -950,7 +941,7 @@ void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPt
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = cluster_config(shape, vDouble, plan.smem, 0, &attr);
         int fit = 0;
-        if (resident_attributes(k, true, plan.smem) == cudaSuccess &&
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
             cudaOccupancyMaxActiveClusters(&fit, k, &cfg) == cudaSuccess && fit > 0)
             return;
         (void)cudaGetLastError();
@@ -959,7 +950,8 @@ void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPt
     if (!plan_for(vDouble, shape, nNodes, rowPtr, colIdx, plan)) plan = PcgResidentPlan();
 }
 
-// The resident form with its plan on the device; shape and smem as ef_pcg_resident_plan returned them
+// The resident form with its plan on the device; shape and smem as ef_pcg_resident_plan returned them (which has
+// allowed the kernel that much shared memory and the cluster's size)
 ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes, const int32_t* rowPtr,
                                  const uint16_t* lcol, const int32_t* haloPtr, const int32_t* haloIdx,
                                  const int32_t* groupPtr, size_t smem, const void* vals, const void* binv,
@@ -969,7 +961,6 @@ ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes,
     void* args[] = {&nNodes, &rowPtr, &lcol, &haloPtr, &haloIdx, &groupPtr, &vals, &binv, &mask, &b, &x, &z,
                     &slots, &copies, &res, &maxIter, &rtol2, &flags};
     const void* k = pcg_resident(vDouble, shape.lpr, shape.cluster);
-    EF_CUDA(resident_attributes(k, shape.cluster, smem));
     ef::note_launches(1);
     if (shape.cluster) {
         cudaLaunchAttribute attr;
