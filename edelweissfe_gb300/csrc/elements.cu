@@ -185,11 +185,11 @@ struct SSShared {
     // per-element rows padded by one entry, so that the elements of a warp fall on different banks
     float2 du[EPB][NN * 3 + 1];       // dU split into FP32 pairs, [3a + i]
     float2 sw[EPB][NQ * 6 + 1];       // sigma w detJ split into FP32 pairs, [6q + i]
-    KT tn[EPB][NQ][9];                // FP32: lt*w, mt*w, c1*w, n[6]; FP64: c2, c1, w (its sign)
+    KT tn[EPB][NQ][9];                // FP32 and FP64 with one Gauss point: lt*w, mt*w, c1*w, n[6]; FP64: c2, c1, w (its sign)
     union {
         float2 g[EPB][NG];            // dN/dx split into FP32 pairs, [(q NN + a) 3 + c] (the FP32 stiffness reads hi)
         struct {                      // the FP64 stiffness, once the residual is done with g
-            double gd[EPB][NG];       // sqrt(|w detJ|) dN/dx
+            double gd[EPB][NG];       // sqrt(|w detJ|) dN/dx (one Gauss point: dN/dx)
             double vd[sizeof(KT) == 8 ? EPB : 1][sizeof(KT) == 8 ? NG : 1];  // n . gd, where plastic
         } d;
     } u;
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
 #pragma unroll
             for (int i = 0; i < 6; ++i) tang[(3 + i) * nQPtot + qi] = mo.c1 != 0.0 ? mo.n[i] : 0.0;
         }
-        if (sizeof(KT) == 8) {
+        if (sizeof(KT) == 8 && NQ > 1) {
             sh.tn[le][q][0] = (KT)mo.c2;
             sh.tn[le][q][1] = (KT)mo.c1;
             sh.tn[le][q][2] = (KT)wdet;
@@ -356,7 +356,55 @@ __global__ void __launch_bounds__(SSShared<NN, NQ, KT>::BLOCK, sizeof(KT) == 8 ?
     // plastic branch is then rarely taken for some of its lanes only) and 36 pairs an element leave no lanes idle (10,240
     // hex8 J2 elements in FP64 312 -> 292 us, 160,000 in FP32, where the FP64 constitutive update bounds it, 478 -> 474)
     const int nItems = min(EPB, nEl - (int)blockIdx.x * EPB) * NP;
-    if constexpr (sizeof(KT) == 8) {
+    if constexpr (sizeof(KT) == 8 && NQ == 1) {
+        // ---- stiffness of one Gauss point in FP64: there is nothing to sum, so the three terms are formed per pair, 30
+        // instructions and 12 more where plastic (as sums of outer products 30 and 60), from the FP64 gradients and va,
+        // which the element's lanes make by nodes.  C3D8R J2 elements, us with both formed per pair from the split
+        // geometry, as sums of outer products and now: 10,240 135, 150 and 88, 54,000 514, 587 and 306
+        __syncthreads();  // the residual has read g
+        for (int a = valid ? lane : NN; a < NN; a += TPE) {
+            const double* gq = geo + (int64_t)e * (3 * NN + 1) + 3 * a;
+            const double g0 = gq[0], g1 = gq[1], g2 = gq[2];
+            double* gd = &sh.u.d.gd[le][3 * a];
+            gd[0] = g0;
+            gd[1] = g1;
+            gd[2] = g2;
+            const KT* tn = sh.tn[le][0];
+            if (tn[2] != 0.0) {
+                double* vd = &sh.u.d.vd[le][3 * a];
+                vd[0] = fma(tn[7], g2, fma(tn[6], g1, tn[3] * g0));
+                vd[1] = fma(tn[8], g2, fma(tn[4], g1, tn[6] * g0));
+                vd[2] = fma(tn[5], g2, fma(tn[8], g1, tn[7] * g0));
+            }
+        }
+        __syncthreads();
+        for (int item = tid; item < nItems; item += SSShared<NN, NQ, KT>::BLOCK) {
+            const int le = item / NP, p = item - le * NP;
+            const int a = pair_a(p, NN);
+            const int b = a + (p - (a * NN - a * (a - 1) / 2));
+            const KT* tn = sh.tn[le][0];
+            const double *ga = &sh.u.d.gd[le][3 * a], *gb = &sh.u.d.gd[le][3 * b];
+            const double lt = tn[0], mt = tn[1], c1 = tn[2];
+            const double la[3] = {lt * ga[0], lt * ga[1], lt * ga[2]}, mb[3] = {mt * gb[0], mt * gb[1], mt * gb[2]};
+            const double s = fma(ga[2], mb[2], fma(ga[1], mb[1], ga[0] * mb[0]));
+            KT k[3][3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) k[i][j] = fma(la[i], gb[j], i == j ? fma(mb[i], ga[j], s) : mb[i] * ga[j]);
+            if (MAT == MAT_VON_MISES && c1 != 0.0) {
+                const double *va = &sh.u.d.vd[le][3 * a], *vb = &sh.u.d.vd[le][3 * b];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const double cv = c1 * va[i];
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) k[i][j] = fma(-cv, vb[j], k[i][j]);
+                }
+            }
+            store(blockIdx.x * EPB + le, p, a, b, k);
+        }
+        return;
+    } else if constexpr (sizeof(KT) == 8) {
         // ---- stiffness in FP64, which the FP64 pipe bounds: K_ab = sum_q lt ga(x)gb + mt (gb(x)ga + ga.gb I)
         // - c1 va(x)vb with lt = lam + c2/3, mt = G - c2/2 and lam, G of the element, so that
         //   K = lam A + G (A^T + tr A I) + B/3 - (B^T + tr B I)/2 - V,
