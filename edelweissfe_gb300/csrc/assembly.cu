@@ -165,7 +165,8 @@ __device__ __forceinline__ double vij_value(int k, const CsrGroups& G, const KT*
     return (double)Kblk[blk * 9 + (na <= nb ? 3 * i + j : 3 * j + i)];
 }
 
-template <typename KT, int ND, bool DIRECT>
+// DEAL = false: a thread takes its own slot (csr_deal)
+template <typename KT, int ND, bool DIRECT, bool DEAL>
 __global__ void __launch_bounds__(kCsrThreads) csr_scatter_kernel(int64_t nnz, const int64_t* __restrict__ seg,
                                                                   const int32_t* __restrict__ perm, CsrGroups G,
                                                                   const KT* __restrict__ V, double* __restrict__ data) {
@@ -177,42 +178,45 @@ __global__ void __launch_bounds__(kCsrThreads) csr_scatter_kernel(int64_t nnz, c
     const int64_t s0 = (int64_t)blockIdx.x * kCsrThreads;
     const int64_t t0 = s0 + tid < nnz ? seg[s0 + tid] : 0;
     const int n0 = s0 + tid < nnz ? (int)(seg[s0 + tid + 1] - t0) : 0;
-    start[tid] = (int)t0;  // (fewer than 2^31 VIJ values)
-    len[tid] = n0;
-    const int bucket = min(n0, kCsrBuckets - 1);
-    int rank = 0;
+    int mine = tid;
+    if constexpr (DEAL) {
+        start[tid] = (int)t0;  // (fewer than 2^31 VIJ values)
+        len[tid] = n0;
+        const int bucket = min(n0, kCsrBuckets - 1);
+        int rank = 0;
 #pragma unroll
-    for (int b = 0; b < kCsrBuckets; ++b) {
-        const unsigned m = __ballot_sync(0xffffffffu, bucket == b);
-        if (bucket == b) rank = __popc(m & ((1u << lane) - 1));
-        if (lane == 0) first[w][b] = __popc(m);
-    }
-    __syncthreads();
-    if (w == 0) {  // exclusive sums over (bucket, warp)
-        int tot = 0;
-        if (lane < kCsrBuckets)
-            for (int q = 0; q < kCsrThreads / 32; ++q) tot += first[q][lane];
-        int base = tot;
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, base, o);
-            if (lane >= o) base += v;
+        for (int b = 0; b < kCsrBuckets; ++b) {
+            const unsigned m = __ballot_sync(0xffffffffu, bucket == b);
+            if (bucket == b) rank = __popc(m & ((1u << lane) - 1));
+            if (lane == 0) first[w][b] = __popc(m);
         }
-        base -= tot;
-        if (lane < kCsrBuckets)
-            for (int q = 0; q < kCsrThreads / 32; ++q) {
-                const int c = first[q][lane];
-                first[q][lane] = base;
-                base += c;
+        __syncthreads();
+        if (w == 0) {  // exclusive sums over (bucket, warp)
+            int tot = 0;
+            if (lane < kCsrBuckets)
+                for (int q = 0; q < kCsrThreads / 32; ++q) tot += first[q][lane];
+            int base = tot;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, base, o);
+                if (lane >= o) base += v;
             }
+            base -= tot;
+            if (lane < kCsrBuckets)
+                for (int q = 0; q < kCsrThreads / 32; ++q) {
+                    const int c = first[q][lane];
+                    first[q][lane] = base;
+                    base += c;
+                }
+        }
+        __syncthreads();
+        order[first[w][bucket] + rank] = (unsigned char)tid;
+        __syncthreads();
+        mine = order[tid];
     }
-    __syncthreads();
-    order[first[w][bucket] + rank] = (unsigned char)tid;
-    __syncthreads();
-    const int mine = order[tid];
     if (s0 + mine >= nnz) return;
-    const int n = len[mine];
-    const int32_t* pk = perm + start[mine];
+    const int n = DEAL ? len[mine] : n0;
+    const int32_t* pk = perm + (DEAL ? start[mine] : (int)t0);
     double acc = 0.0;
     for (int t = 0; t < n; t += 4) {
         double v[4];
@@ -431,11 +435,16 @@ ef_status ef_launch_vij_export(int nEl, int nn, int np, const void* Kblk, int kD
     return EF_OK;
 }
 
-ef_status ef_launch_csr_scatter(int64_t nnz, const int64_t* seg, const int32_t* perm, const double* V, double* data,
-                                cudaStream_t s) {
+// Dealing a CTA's slots out by count pays where they have many values: of a VIJ vector us without and with at
+// 2.3 values a slot (10,240 hex8 elements) 58.8 and 51.2, at 1.95 (125 hex8) 16.8 and 15.6, at 1.64 (2,880 hex20) 77.0 and
+// 88.2, at 1.58 (546 hex20) 24.2 and 26.5
+static bool csr_deal(int64_t nVIJ, int64_t nnz) { return 10 * nVIJ > 17 * nnz; }
+
+ef_status ef_launch_csr_scatter(int64_t nVIJ, int64_t nnz, const int64_t* seg, const int32_t* perm, const double* V,
+                                double* data, cudaStream_t s) {
     if (nnz == 0) return EF_OK;
-    csr_scatter_kernel<double, 0, false><<<nblk(nnz, kCsrThreads), kCsrThreads, 0, ef::counted(s)>>>(nnz, seg, perm,
-                                                                                                  CsrGroups{}, V, data);
+    auto k = csr_deal(nVIJ, nnz) ? csr_scatter_kernel<double, 0, false, true> : csr_scatter_kernel<double, 0, false, false>;
+    k<<<nblk(nnz, kCsrThreads), kCsrThreads, 0, ef::counted(s)>>>(nnz, seg, perm, CsrGroups{}, V, data);
     EF_CUDA(cudaGetLastError());
     return EF_OK;
 }
@@ -445,7 +454,7 @@ ef_status ef_launch_csr_from_blocks(int64_t nnz, const int64_t* seg, const int32
     if (nnz == 0) return EF_OK;
     const int nd = G.n == 1 ? G.nd[0] : 0;
 #define EF_CSR(T_, N_)                                                                                            \
-    csr_scatter_kernel<T_, N_, true><<<nblk(nnz, kCsrThreads), kCsrThreads, 0, ef::counted(s)>>>(nnz, seg, perm, G, \
+    csr_scatter_kernel<T_, N_, true, true><<<nblk(nnz, kCsrThreads), kCsrThreads, 0, ef::counted(s)>>>(nnz, seg, perm, G, \
                                                                                                (const T_*)Kblk, data)
     if (kDouble) {
         if (nd == 24)

@@ -191,8 +191,8 @@ ef_status ef_launch_vij_export(int nEl, int nn, int np, const void* Kblk, int kD
 ef_status ef_launch_results_gather(int64_t nPts, int nQ, int nQP, int64_t nq, int first, int count,
                                    const int32_t* elements, const int32_t* qps, const double* state, double* table,
                                    cudaStream_t s);
-ef_status ef_launch_csr_scatter(int64_t nnz, const int64_t* seg, const int32_t* perm, const double* V, double* data,
-                                cudaStream_t s);
+ef_status ef_launch_csr_scatter(int64_t nVIJ, int64_t nnz, const int64_t* seg, const int32_t* perm, const double* V,
+                                double* data, cudaStream_t s);
 ef_status ef_launch_csr_from_blocks(int64_t nnz, const int64_t* seg, const int32_t* perm, const ef::CsrGroups& G,
                                     const void* Kblk, int kDouble, double* data, cudaStream_t s);
 ef_status ef_launch_csr_dirichlet_rows(int64_t nRows, const int64_t* rows, const int32_t* indptr,

@@ -44,7 +44,7 @@ ef_status ef_update_csr(ef_ctx* c, const double* Kvij, double* csrData, void* st
         }
         return ef_launch_csr_from_blocks(c->nnz, c->dCsrSeg, c->dCsrPerm, G, c->Kblk, c->keFp64, csrData, s);
     }
-    return ef_launch_csr_scatter(c->nnz, c->dCsrSeg, c->dCsrPerm, Kvij, csrData, s);
+    return ef_launch_csr_scatter(c->nVIJ, c->nnz, c->dCsrSeg, c->dCsrPerm, Kvij, csrData, s);
 }
 
 ef_status ef_csr_dirichlet_rows(ef_ctx* c, double* csrData, const int64_t* rows, int64_t nRows, void* stream) {
