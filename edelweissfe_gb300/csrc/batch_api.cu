@@ -70,6 +70,7 @@ static ef_status batch_plans(ef_ctx* c, int nProb, const int32_t* nodePtr) {
     std::vector<int> sizes(nProb);
     for (int p = 0; p < nProb; ++p) sizes[p] = nodePtr[p + 1] - nodePtr[p];
     c->batchCluster = ef_batch_cluster_size(c->nSM, sizes);
+    if (!c->batchTileSet) c->batchTile = ef_batch_default_tile(nProb, c->nNodes);
     return EF_OK;
 }
 
@@ -124,6 +125,7 @@ ef_status ef_batch_set_tile(ef_ctx* c, int tile) {
         return EF_ERR_ARG;
     }
     c->batchTile = tile;
+    c->batchTileSet = true;
     return EF_OK;
 }
 
@@ -190,6 +192,7 @@ ef_status ef_batch_autotune(ef_ctx* c, double rtol, int maxIter, const double* b
         }
     }
     c->batchTile = bestT;
+    c->batchTileSet = true;
     if (tileOut) *tileOut = bestT;
     return EF_OK;
 }

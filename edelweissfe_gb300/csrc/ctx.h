@@ -577,7 +577,8 @@ struct ef_ctx {
     // batch of independent problems (contiguous node ranges), see ef_batch_setup
     int batchN = 0;
     int32_t *dBatchNodePtr = nullptr, *dBatchOrder = nullptr;
-    int batchTile = 6;  // index into the batched-PCG tile shapes
+    int batchTile = 6;          // index into the batched-PCG tile shapes
+    bool batchTileSet = false;  // by the caller or the autotuner (else ef_batch_setup takes the default)
     int batchCluster = 1;                                // CTAs per problem
     BatchPlanDev batchPlan[3];                           // sliced copies for 1, 4 and 8 lanes per row (one buffer)
     std::vector<void*> batchMem;                         // their device arrays

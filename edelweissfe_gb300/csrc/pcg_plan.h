@@ -25,6 +25,12 @@ struct PcgResidentPlan {
 void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPtr, const int32_t* colIdx,
                           PcgResidentPlan& plan);
 
+// The batched PCG's tile shape (an index into kBatchTiles) before any tuning: 512 threads with 4 lanes per row, or 128 for batches of small problems, whose rows leave
+// most of 512 threads idle at every barrier.  us of a solve with 128 and 512 threads: 2,000 problems of 8 nodes 133 and
+// 343, 1,000 of 27 537 and 1,055, 500 of 64 796 and 1,159, 100 of 64 348 and 315, 152 of 125 888 and 686, 152 of 343
+// 4,707 and 2,423
+inline int ef_batch_default_tile(int64_t nProb, int64_t nNodes) { return nNodes <= 64 * nProb ? 1 : 6; }
+
 // The batched PCG's sliced copy for one number of lanes per block row: device arrays
 struct BatchPlanDev {
     int nGroups = 0;                       // groups of 32 / lanes rows, none across two problems
