@@ -92,11 +92,14 @@ __device__ __forceinline__ bool batch_sum(const double (&v)[NV], int count, Batc
 // block in nine planes of 32 values, so that a warp's loads are contiguous (from the block rows they
 // touch 18 lines each).  Up to 512 threads' worth of registers (128 a thread) keep two steps of loads in
 // flight; with 64 the same shapes took a fifth longer.  MULTI: clusters of more than one CTA; p is then gathered through L2.
-template <int TPB, int LPR, bool MULTI>
+// SLICED = false: no memory for the sliced copy; the blocks are read from the block rows themselves, lane l's j-th
+// block in the same order (the same sums; ms of a solve with the copy and without: one cube of 8 elements an edge 1.44 and
+// 1.59, 160 of 4..16 33.0 and 33.5, with one lane per row 66.5 and 89.9).
+template <int TPB, int LPR, bool MULTI, bool SLICED>
 __global__ void __launch_bounds__(TPB, 512 / TPB) batched_pcg_kernel(
     int nProb, const int32_t* __restrict__ nodePtr, const int32_t* __restrict__ order,
-    const int32_t* __restrict__ groupBase, const int32_t* __restrict__ groupPtr, const int32_t* __restrict__ col,
-    const double* __restrict__ vals, const double* __restrict__ binv, const uint8_t* __restrict__ mask,
+    const int32_t* __restrict__ groupBase, const int32_t* __restrict__ groupPtr, const int32_t* __restrict__ rowPtr,
+    const int32_t* __restrict__ col, const double* __restrict__ vals, const double* __restrict__ binv, const uint8_t* __restrict__ mask,
     const double* __restrict__ b, double* x, double* rA, double* rB, double* z, double* p, double* q, int maxIter,
     double rtol2, int* __restrict__ itersOut, double* __restrict__ relOut, int* ticket) {
     constexpr int RPW = 32 / LPR;  // rows of a group
@@ -161,15 +164,17 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) batched_pcg_kernel(
             double pq[1] = {0.0};
             for (int g = g0 + warp; g < g1; g += TPB / 32) {
                 const int m = n0 + g * RPW + lane / LPR;
-                const int j1 = gp[g + 1];
+                // block j of the lane: step j of the sliced copy, or entry j of the block row
+                const int j0 = SLICED ? gp[g] : (m < r1 ? rowPtr[m] + l : 0);
+                const int j1 = SLICED ? gp[g + 1] : (m < r1 ? rowPtr[m + 1] : 0);
                 double y0 = 0.0, y1 = 0.0, y2 = 0.0;
 #pragma unroll 2
-                for (int j = gp[g]; j < j1; ++j) {
-                    const double* v = vals + (int64_t)288 * j + lane;
-                    const double* pv = p + 3 * (int64_t)__ldg(col + 32 * (int64_t)j + lane);
+                for (int j = j0; j < j1; j += SLICED ? 1 : LPR) {
+                    const double* v = vals + (SLICED ? (int64_t)288 * j + lane : (int64_t)9 * j);
+                    const double* pv = p + 3 * (int64_t)__ldg(col + (SLICED ? 32 * (int64_t)j + lane : (int64_t)j));
                     double a[9];
 #pragma unroll
-                    for (int i = 0; i < 9; ++i) a[i] = __ldg(v + 32 * i);
+                    for (int i = 0; i < 9; ++i) a[i] = __ldg(v + (SLICED ? 32 * i : i));
                     const double p0 = MULTI ? __ldcg(pv) : pv[0], p1 = MULTI ? __ldcg(pv + 1) : pv[1],
                                  p2 = MULTI ? __ldcg(pv + 2) : pv[2];
                     block_fma(a, p0, p1, p2, y0, y1, y2);
@@ -308,12 +313,12 @@ __global__ void __launch_bounds__(256) batch_norms_kernel(int nProb, const int32
     }
 }
 
-template <int TPB, int LPR, bool MULTI>
-static ef_status launch_batched(const BatchPlanDev& pl, int cluster, int nSM, int nProb, const double* binv,
-                                const uint8_t* mask, const double* b, double* x, double* r, double* r2, double* z,
+template <int TPB, int LPR, bool MULTI, bool SLICED>
+static ef_status launch_batched(const BatchPlanDev& pl, int cluster, int nSM, int nProb, const int32_t* rowPtr,
+                                const int32_t* col, const double* vals, const double* binv, const uint8_t* mask, const double* b, double* x, double* r, double* r2, double* z,
                                 double* p, double* q, int maxIter, double rtol2, int* iters, double* rel, int* ticket,
                                 cudaStream_t s) {
-    auto k = batched_pcg_kernel<TPB, LPR, MULTI>;
+    auto k = batched_pcg_kernel<TPB, LPR, MULTI, SLICED>;
     int perSM = 0;
     EF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, TPB, 0));
     // as many clusters as are resident at once; a cluster that is scheduled later finds the list empty
@@ -329,9 +334,8 @@ static ef_status launch_batched(const BatchPlanDev& pl, int cluster, int nSM, in
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    EF_CUDA(cudaLaunchKernelEx(&cfg, k, nProb, pl.nodePtr, pl.order, pl.groupBase, pl.groupPtr, (const int32_t*)pl.col,
-                               (const double*)pl.vals, binv, mask, b, x, r, r2, z, p, q, maxIter, rtol2, iters, rel,
-                               ticket));
+    EF_CUDA(cudaLaunchKernelEx(&cfg, k, nProb, pl.nodePtr, pl.order, pl.groupBase, pl.groupPtr, rowPtr, col, vals, binv, mask,
+                               b, x, r, r2, z, p, q, maxIter, rtol2, iters, rel, ticket));
     return EF_OK;
 }
 
@@ -379,17 +383,19 @@ ef_status ef_launch_batched_pcg(int tile, const BatchPlanDev& pl, int cluster, i
                                 int maxIter, double rtol2, int* iters, double* rel, int* ticket, cudaStream_t s) {
     if (nProb == 0) return EF_OK;
     const int sliceGrid = std::max(1, std::min((pl.nGroups + 7) / 8, 16 * nSM));
+    const bool sliced = pl.vals != nullptr;
+#define EF_BT_LAUNCH(T, L, M, S)                                                                                      \
+    launch_batched<T, L, M, S>(pl, cluster, nSM, nProb, rowPtr, S ? pl.col : colIdx, S ? pl.vals : bsr, binv, mask, b, x, \
+                               r, r2, z, p, q, maxIter, rtol2, iters, rel, ticket, s)
 #define EF_BT(T, L)                                                                                                   \
     do {                                                                                                              \
-        if (pl.nGroups > 0)                                                                                           \
+        if (sliced && pl.nGroups > 0)                                                                                 \
             batch_slice_kernel<L><<<sliceGrid, 256, 0, ef::counted(s)>>>(pl.nGroups, pl.groupRow, pl.groupEnd,        \
                                                                          pl.groupStep, rowPtr, colIdx, bsr, pl.vals,  \
                                                                          pl.col);                                     \
         EF_CUDA(cudaGetLastError());                                                                                  \
-        return cluster > 1 ? launch_batched<T, L, true>(pl, cluster, nSM, nProb, binv, mask, b, x, r, r2, z, p, q,    \
-                                                        maxIter, rtol2, iters, rel, ticket, s)                        \
-                           : launch_batched<T, L, false>(pl, 1, nSM, nProb, binv, mask, b, x, r, r2, z, p, q, maxIter, \
-                                                         rtol2, iters, rel, ticket, s);                               \
+        if (cluster > 1) return sliced ? EF_BT_LAUNCH(T, L, true, true) : EF_BT_LAUNCH(T, L, true, false);            \
+        return sliced ? EF_BT_LAUNCH(T, L, false, true) : EF_BT_LAUNCH(T, L, false, false);                           \
     } while (0)
     switch (tile) {
         case 0: EF_BT(128, 1);
@@ -404,6 +410,7 @@ ef_status ef_launch_batched_pcg(int tile, const BatchPlanDev& pl, int cluster, i
             return EF_ERR_ARG;
     }
 #undef EF_BT
+#undef EF_BT_LAUNCH
 }
 
 ef_status ef_launch_batch_norms(int nProb, const int32_t* nodePtr, const double* R, const double* F, const double* D,

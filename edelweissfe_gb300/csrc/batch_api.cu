@@ -54,12 +54,20 @@ static ef_status batch_plans(ef_ctx* c, int nProb, const int32_t* nodePtr) {
         most = std::max(most, steps);
     }
     ef_status st = EF_OK;
-    double* vals = dalloc<double>((size_t)288 * most, &st);
-    if (!vals) return st;
-    c->batchMem.push_back(vals);
-    int32_t* col = dalloc<int32_t>((size_t)32 * most, &st);
-    if (!col) return st;
-    c->batchMem.push_back(col);
+    // the copy takes as much as the system itself and its padding; where there is no room for it (or with EF_BATCH_SLICED=0),
+    // the kernels read the block rows
+    const char* e = getenv("EF_BATCH_SLICED");
+    double* vals = e && atoi(e) == 0 ? nullptr : dalloc<double>((size_t)288 * most, &st);
+    int32_t* col = vals ? dalloc<int32_t>((size_t)32 * most, &st) : nullptr;
+    if (!col) {
+        cudaFree(vals);
+        (void)cudaGetLastError();
+        vals = nullptr;
+        st = EF_OK;
+    } else {
+        c->batchMem.push_back(vals);
+        c->batchMem.push_back(col);
+    }
     c->dBatchTicket = dalloc<int>(1, &st);
     if (!c->dBatchTicket) return st;
     c->batchMem.push_back(c->dBatchTicket);

@@ -41,6 +41,6 @@ struct BatchPlanDev {
     const int32_t *groupRow = nullptr;     // [groups] first row
     const int32_t *groupEnd = nullptr;     // [groups] the problem's end row
     const int32_t *groupStep = nullptr;    // [groups][2] first and last step
-    double* vals = nullptr;                // [steps][9][32]
+    double* vals = nullptr;                // [steps][9][32] (null: no copy)
     int32_t* col = nullptr;                // [steps][32]
 };

@@ -287,7 +287,10 @@ ef_status ef_set_group_cutback(ef_ctx* ctx, int groupId, double scale);
 ef_status ef_set_group_props(ef_ctx* ctx, int groupId, const double* table, int nRows, int nProps,
                              const int32_t* elemRow);
 /* Declares the problems: problem p owns the nodes [nodePtr[p], nodePtr[p+1]) (host int32
- * [nProb+1], covering all nodes); no 3x3 block may couple two problems.  Needs EF_OPT_KE_FP64. */
+ * [nProb+1], covering all nodes); no 3x3 block may couple two problems.  Needs EF_OPT_KE_FP64.
+ * Allocates a second copy of the FP64 blocks in the solve kernel's order (1.1 to 1.5 times their
+ * size for cubes of 20 to 4 elements an edge, more for smaller problems); where the device has no room for
+ * it, the solves read the blocks themselves. */
 ef_status ef_batch_setup(ef_ctx* ctx, int nProb, const int32_t* nodePtr);
 /* Tile shapes of the batched PCG: tile t in [0, ef_batch_tile_count()) runs CTAs of threadsPerCta
  * threads with lanesPerRow lanes per 3x3 block row in the matrix products.  A problem is solved by a

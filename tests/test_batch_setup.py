@@ -60,3 +60,23 @@ def test_untuned_tile_follows_the_problem_size(gpu_lib, sizes, tile):
     y = _solve(s, b)
     _lib.check(s.lib.ef_batch_setup(s.ctx, s.nProb, s.nodePtr.ctypes.data), "ef_batch_setup")
     assert torch.equal(y, _solve(s, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[5], [1, 2, 9, 3, 6], [14] + [2] * 30, [3, 4, 5, 6] * 100], ids=["lone", "few", "uneven", "many"])
+def test_solves_without_the_sliced_copy(gpu_lib, monkeypatch, sizes):
+    """A batch whose sliced copy finds no room (EF_BATCH_SLICED=0 stands in for it) is solved from the block rows, with every
+    tile and cluster size, by the same sums."""
+    from edelweissfe_gb300 import _lib
+
+    s, b = _batch(sizes)
+    for tile in range(gpu_lib.ef_batch_tile_count()):
+        _lib.check(s.lib.ef_batch_set_tile(s.ctx, tile), "ef_batch_set_tile")
+        with monkeypatch.context() as env:
+            x = _solve(s, b)
+            env.setenv("EF_BATCH_SLICED", "0")
+            free = torch.cuda.mem_get_info()[0]
+            _lib.check(s.lib.ef_batch_setup(s.ctx, s.nProb, s.nodePtr.ctypes.data), "ef_batch_setup")
+            assert torch.cuda.mem_get_info()[0] >= free
+            assert torch.equal(x, _solve(s, b))
+        _lib.check(s.lib.ef_batch_setup(s.ctx, s.nProb, s.nodePtr.ctypes.data), "ef_batch_setup")
