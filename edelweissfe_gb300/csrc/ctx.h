@@ -242,16 +242,9 @@ extern thread_local long long* t_captureCount;
 
 namespace efh {
 
-struct PcgResultHost {
-    int iterations;
-    int status;
-    double rr;
-    double bb;
-};
-
 struct HostResults {
     double red[8];   // reductions
-    PcgResultHost pcg;
+    PcgResult pcg;
     int flags[2];    // copy of the context's device flags
 };
 
@@ -612,7 +605,7 @@ struct ef_ctx {
 // system.cu
 ef_status residual64(ef_ctx* c, const double* x, const double* b, double* r, double* rr, cudaStream_t s);
 ef_status dot_host(ef_ctx* c, const double* a, const double* b, double* out, cudaStream_t s);
-ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol, PcgResultHost* out,
+ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol, PcgResult* out,
                   ef_solve_info* prof, cudaStream_t s);
 // precond.cu
 ef_status amg_workspace(ef_ctx* c);

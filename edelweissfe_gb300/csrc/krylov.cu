@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <vector>
 
 #include "cluster.cuh"
@@ -102,13 +103,6 @@ __global__ void __launch_bounds__(kKB) bsr_residual_kernel(int nNodes, const int
     }
 }
 
-struct PcgResult {
-    int iterations;
-    int status;
-    double rr;   // final squared residual norm
-    double bb;   // squared RHS norm
-};
-
 // ---- block-Jacobi PCG, persistent over all iterations ------------------------------------------
 //
 // What bounds an iteration is latency, not bandwidth: the systems it runs on (up to some ten
@@ -131,6 +125,13 @@ constexpr int kPcgMaxCtas = 160;                    // slots of a reduction (one
 constexpr int kPcgMaxCluster = 16;                  // CTAs of the cluster form
 constexpr int kPcgPoll = kPcgMaxCtas / 32;          // slots a lane of the polling warp watches
 constexpr unsigned kPcgSpinLimit = 1u << 22;        // polls before a barrier gives up (seconds)
+
+// Where a launch reports to, and how often a barrier polls
+struct PcgWait {
+    PcgResult* res;
+    int* flags;
+    unsigned limit;
+};
 constexpr unsigned long long kPcgEmpty = ~0ull;     // an unwritten slot (a NaN that no sum produces)
 constexpr size_t kPcgSlotBytes = sizeof(double) * 3 * 2 * kPcgMaxCtas;
 
@@ -181,10 +182,10 @@ struct PcgShared {
 // Few CTAs poll one set of slots: with all 152 on the same lines a reduction takes 1 us longer, so a CTA
 // stores into `copies` sets and polls one of them.
 // CL: the grid is one cluster; the sums go into every CTA's shared memory, behind the cluster's barrier.
-// Returns sh.go: -1 when a CTA did not arrive within the poll limit (EF_FLAG_BARRIER is set).
+// Returns sh.go: -1 when a CTA did not arrive within the poll limit (EF_FLAG_BARRIER and res->gaveUp are set).
 template <typename VT, int TPB, int NV, bool PUB, bool CL, typename F>
 __device__ __forceinline__ int grid_sum(const VT (&v)[NV], int slot, int count, PcgShared<VT, TPB>& sh,
-                                        double* __restrict__ slots, int copies, int& epoch, int* flags, F next) {
+                                        double* __restrict__ slots, int copies, int& epoch, const PcgWait& wait, F next) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (sizeof(VT) == 4) {
 #pragma unroll
@@ -222,7 +223,7 @@ __device__ __forceinline__ int grid_sum(const VT (&v)[NV], int slot, int count, 
 #pragma unroll
             for (int i = 0; i < kPcgPoll; ++i) u[i] = v2[i] = lane + 32 * i < n ? kPcgEmpty : 0ull;
             bool all = false;
-            for (unsigned spin = 0; !all && spin < kPcgSpinLimit; ++spin) {
+            for (unsigned spin = 0; !all && spin < wait.limit; ++spin) {
                 all = true;
 #pragma unroll
                 for (int i = 0; i < kPcgPoll; ++i)
@@ -245,7 +246,10 @@ __device__ __forceinline__ int grid_sum(const VT (&v)[NV], int slot, int count, 
 #pragma unroll
                 for (int j = 0; j < NV; ++j) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
             if (lane == 0) {
-                if (!arrived) atomicOr(flags, EF_FLAG_BARRIER);
+                if (!arrived) {
+                    atomicOr(wait.flags, EF_FLAG_BARRIER);
+                    wait.res->gaveUp = 1;
+                }
                 sh.go = !arrived ? -1 : (next(t) ? 1 : 0);
             }
         }
@@ -284,7 +288,7 @@ template <typename VT, int LPR>
 __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_persistent_kernel(
     int nNodes, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ colIdx, const VT* __restrict__ vals,
     const VT* __restrict__ binv, const uint8_t* __restrict__ mask, const VT* __restrict__ b, VT* x, VT* r, VT* z,
-    VT* pA, VT* pB, VT* q, double* slots, int copies, PcgResult* res, int maxIter, double rtol2, int* flags) {
+    VT* pA, VT* pB, VT* q, double* slots, int copies, PcgWait wait, int maxIter, double rtol2) {
     constexpr int TPB = PcgTpb<VT>::value;
     constexpr int RPI = TPB / LPR;                    // rows per pass of the product
     constexpr int NB = LPR >= 32 ? 1 : (LPR == 16 ? 2 : 4);  // blocks per lane whose loads are issued together
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_persistent_kernel(
             loc[1] += rv[i] * rv[i];
         }
     }
-    int go = grid_sum<VT, TPB, 2, true, false>(loc, slotB, countB, sh, slots, copies, epoch, flags, [&](const double(&t)[2]) {
+    int go = grid_sum<VT, TPB, 2, true, false>(loc, slotB, countB, sh, slots, copies, epoch, wait, [&](const double(&t)[2]) {
         return sca.start(t, rtol2, sh.scalar);
     });
     if (go < 0) return;
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_persistent_kernel(
                     pq[0] += pd * yy;
                 }
             }
-            go = grid_sum<VT, TPB, 1, true, false>(pq, slotA, countA, sh, slots, copies, epoch, flags, [&](const double(&t)[1]) {
+            go = grid_sum<VT, TPB, 1, true, false>(pq, slotA, countA, sh, slots, copies, epoch, wait, [&](const double(&t)[1]) {
                 return sca.step(t, sh.scalar);
             });
             if (go < 0) return;
@@ -407,7 +411,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_persistent_kernel(
                     l2[1] += rv[i] * rv[i];
                 }
             }
-            go = grid_sum<VT, TPB, 2, true, false>(l2, slotB, countB, sh, slots, copies, epoch, flags, [&](const double(&t)[2]) {
+            go = grid_sum<VT, TPB, 2, true, false>(l2, slotB, countB, sh, slots, copies, epoch, wait, [&](const double(&t)[2]) {
                 return sca.direction(t, sh.scalar);
             });
             if (go < 0) return;
@@ -422,10 +426,10 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_persistent_kernel(
         if (k >= maxIter && sca.status == EF_OK && !sca.finished()) sca.status = EF_NOT_CONVERGED;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        res->iterations = k;
-        res->status = sca.status;
-        res->rr = sca.rr;
-        res->bb = sca.bb;
+        wait.res->iterations = k;
+        wait.res->status = sca.status;
+        wait.res->rr = sca.rr;
+        wait.res->bb = sca.bb;
     }
 }
 
@@ -471,7 +475,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
     const int32_t* __restrict__ haloPtr, const int32_t* __restrict__ haloIdx, const int32_t* __restrict__ groupPtr,
     const VT* __restrict__ vals,
     const VT* __restrict__ binv, const uint8_t* __restrict__ mask, const VT* __restrict__ b, VT* __restrict__ x,
-    VT* z, double* slots, int copies, PcgResult* res, int maxIter, double rtol2, int* flags) {
+    VT* z, double* slots, int copies, PcgWait wait, int maxIter, double rtol2) {
     constexpr int TPB = PcgTpb<VT>::value;
     constexpr int RPI = TPB / LPR;
     constexpr int RPW = 32 / LPR;  // rows per warp
@@ -548,7 +552,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
     };
     VT loc[2] = {(VT)0, (VT)0};
     for (int d = tid; d < 3 * rows; d += TPB) update(d, (VT)0, sr, sr2, loc);  // q = 0: r = b
-    int go = grid_sum<VT, TPB, 2, true, CL>(loc, slotB, countB, sh, slots, copies, epoch, flags, [&](const double(&t)[2]) {
+    int go = grid_sum<VT, TPB, 2, true, CL>(loc, slotB, countB, sh, slots, copies, epoch, wait, [&](const double(&t)[2]) {
         return sca.start(t, rtol2, sh.scalar);
     });
     if (go < 0) return;
@@ -586,7 +590,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
                     pq[0] += sp[d] * yy;
                 }
             }
-            go = grid_sum<VT, TPB, 1, false, CL>(pq, slotA, countA, sh, slots, copies, epoch, flags, [&](const double(&t)[1]) {
+            go = grid_sum<VT, TPB, 1, false, CL>(pq, slotA, countA, sh, slots, copies, epoch, wait, [&](const double(&t)[1]) {
                 return sca.step(t, sh.scalar);
             });
             if (go < 0) return;
@@ -600,7 +604,7 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
                 sx[d] += alpha * sp[d];
                 update(d, alpha, sr, sr2, l2);
             }
-            go = grid_sum<VT, TPB, 2, true, CL>(l2, slotB, countB, sh, slots, copies, epoch, flags, [&](const double(&t)[2]) {
+            go = grid_sum<VT, TPB, 2, true, CL>(l2, slotB, countB, sh, slots, copies, epoch, wait, [&](const double(&t)[2]) {
                 return sca.direction(t, sh.scalar);
             });
             if (go < 0) return;
@@ -614,10 +618,10 @@ __global__ void __launch_bounds__(PcgTpb<VT>::value, 1) pcg_resident_kernel(
     if (CL) cluster_barrier();  // no CTA leaves while another may still read its shared memory
     for (int i = tid; i < 3 * rows; i += TPB) x[3 * (int64_t)r0 + i] = sx[i];
     if (blockIdx.x == 0 && tid == 0) {
-        res->iterations = k;
-        res->status = sca.status;
-        res->rr = sca.rr;
-        res->bb = sca.bb;
+        wait.res->iterations = k;
+        wait.res->status = sca.status;
+        wait.res->rr = sca.rr;
+        wait.res->bb = sca.bb;
     }
 }
 
@@ -851,6 +855,12 @@ void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPt
     if (!plan_for(vDouble, shape, nNodes, rowPtr, colIdx, plan)) plan = PcgResidentPlan();
 }
 
+// EF_PCG_POLLS: another limit, for the tests of a wait that runs out
+static PcgWait pcg_wait(void* res, int* flags) {
+    const char* e = getenv("EF_PCG_POLLS");
+    return PcgWait{(PcgResult*)res, flags, e ? (unsigned)strtoul(e, nullptr, 10) : kPcgSpinLimit};
+}
+
 // The resident form with its plan on the device; shape and smem as ef_pcg_resident_plan returned them (which has
 // allowed the kernel that much shared memory and the cluster's size)
 ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes, const int32_t* rowPtr,
@@ -859,8 +869,9 @@ ef_status ef_launch_pcg_resident(int vDouble, const PcgShape& shape, int nNodes,
                                  const uint8_t* mask, const void* b, void* x, void* z, double* slots, void* res,
                                  int maxIter, double rtol2, int* flags, cudaStream_t s) {
     int copies = shape.copies;
+    PcgWait wait = pcg_wait(res, flags);
     void* args[] = {&nNodes, &rowPtr, &lcol, &haloPtr, &haloIdx, &groupPtr, &vals, &binv, &mask, &b, &x, &z,
-                    &slots, &copies, &res, &maxIter, &rtol2, &flags};
+                    &slots, &copies, &wait, &maxIter, &rtol2};
     const void* k = pcg_resident(vDouble, shape.lpr, shape.cluster);
     ef::note_launches(1);
     if (shape.cluster) {
@@ -882,8 +893,9 @@ ef_status ef_launch_pcg(int vDouble, int nSM, int nNodes, const int32_t* rowPtr,
     PcgShape shape;
     pcg_shape(vDouble, nNodes, nSM, &shape);
     int copies = std::min(shape.copies, slotSets);
+    PcgWait wait = pcg_wait(res, flags);
     void* args[] = {&nNodes, &rowPtr, &colIdx, &vals, &binv, &mask, &b, &x, &r, &z, &pA, &pB, &q,
-                    &slots, &copies, &res, &maxIter, &rtol2, &flags};
+                    &slots, &copies, &wait, &maxIter, &rtol2};
     EF_CUDA(cudaMemsetAsync(slots, 0xff, copies * kPcgSlotBytes, s));
     ef::note_launches(1);
     EF_CUDA(cudaLaunchCooperativeKernel(pcg_kernel(vDouble, shape.lpr), shape.grid,

@@ -7,6 +7,22 @@
 
 #include <vector>
 
+// What a PCG launch leaves for the host, in memory that the host clears before the launch (pcg_result_clear): the
+// record is CTA 0's, gaveUp any CTA's.  A CTA that gave up waiting for the others leaves its rows of x unwritten, also
+// when CTA 0 has seen the end of the solve.
+struct PcgResult {
+    int iterations;
+    int status;   // -1: not written
+    int gaveUp;
+    double rr;    // final squared residual norm
+    double bb;    // squared RHS norm
+};
+inline void pcg_result_clear(PcgResult& r) {
+    r.status = -1;
+    r.gaveUp = 0;
+}
+inline bool pcg_result_timed_out(const PcgResult& r) { return r.status == -1 || r.gaveUp != 0; }
+
 struct PcgShape {
     int grid = 1, lpr = 32;  // CTAs and lanes per block row
     int copies = 1;          // slot sets of a reduction

@@ -347,7 +347,7 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
         // all-FP64 PCG to the target tolerance (relative to ||b||)
         EF_CUDA(cudaMemcpyAsync(c->w64k[0], r64, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         const double rel = rr > 0.0 ? o->rtol * bnorm / sqrt(rr) : 1.0;
-        PcgResultHost pr;
+        PcgResult pr;
         if (rr > 0.0) {
             EF_CHECK(run_pcg(c, 1, c->w64k[0], c->w64k[1], o->maxIter, std::min(rel, 1.0), &pr, o->profile ? &inf : nullptr, s));
             total = pr.iterations;
@@ -374,7 +374,7 @@ ef_status ef_solve(ef_ctx* c, const ef_solve_opts* o, const double* b, double* x
                                  c->fgPc == EF_FGMRES_PC_MULTIGRID && !c->nnOn;
             const double inner = std::max(floored ? std::max(o->innerRtol, c->refineFloor) : o->innerRtol,
                                           c->refineAim * o->rtol * bnorm / rn);
-            PcgResultHost pr;
+            PcgResult pr;
             if (o->method == EF_SOLVE_FGMRES) {
                 const bool timeSetup = o->profile && (c->sellStale || c->amgStale);
                 if (timeSetup) EF_CUDA(cudaEventRecord(c->ev[0], s));

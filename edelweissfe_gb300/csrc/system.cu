@@ -192,10 +192,10 @@ static ef_status pcg_plan(ef_ctx* c, int vDouble) {
 // one PCG launch on the free DOFs: solves K d = rhs (rhs zero on Dirichlet DOFs); vDouble: the
 // precision of the system
 ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol,
-                         PcgResultHost* out, ef_solve_info* prof, cudaStream_t s) {
+                         PcgResult* out, ef_solve_info* prof, cudaStream_t s) {
     void** w = vDouble ? c->w64k : c->w32;
     EF_CHECK(pcg_plan(c, vDouble));
-    c->hRes->pcg.status = -1;  // stays so when a CTA gave up waiting for the others
+    pcg_result_clear(c->hRes->pcg);
     if (prof) EF_CUDA(cudaEventRecord(c->ev[0], s));
     if (c->pcgSmem > 0)
         EF_CHECK(ef_launch_pcg_resident(vDouble, c->pcgShape, (int)c->nNodes, c->dRowPtr, c->dPcgLcol, c->dPcgHaloPtr,
@@ -214,7 +214,7 @@ ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIte
         prof->kernelMs += ms;
         prof->kernelLaunches += 1;
     }
-    if (out->status == -1) {
+    if (pcg_result_timed_out(*out)) {
         ef_set_error("PCG: grid barrier timed out");
         return EF_ERR_DEVICE;
     }
