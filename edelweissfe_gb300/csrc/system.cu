@@ -57,8 +57,16 @@ ef_status ef_csr_dirichlet_rows(ef_ctx* c, double* csrData, const int64_t* rows,
             return EF_ERR_ARG;
         }
     // the rows go through buffers of the context (no allocation and no synchronisation per call): a pinned copy, so
-    // that the caller's array is free again, and a device one; both wait for the launch that last used them
+    // that the caller's array is free again, and a device one; both wait for the launch that last used them.  Under
+    // stream capture that wait could not be kept (the event would belong to the capture, and a replay would read
+    // whatever rows the pinned copy holds by then), so the call is refused there
     cudaStream_t s = (cudaStream_t)stream;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    EF_CUDA(cudaStreamIsCapturing(s, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        ef_set_error("ef_csr_dirichlet_rows: not under stream capture");
+        return EF_ERR_STATE;
+    }
     if (!c->csrRowsDone) EF_CUDA(cudaEventCreateWithFlags(&c->csrRowsDone, cudaEventDisableTiming));
     EF_CUDA(cudaEventSynchronize(c->csrRowsDone));
     if (c->csrRowsCap < nRows) {
@@ -74,9 +82,9 @@ ef_status ef_csr_dirichlet_rows(ef_ctx* c, double* csrData, const int64_t* rows,
     }
     memcpy(c->hCsrRows, rows, sizeof(int64_t) * nRows);
     EF_CUDA(cudaMemcpyAsync(c->dCsrRows, c->hCsrRows, sizeof(int64_t) * nRows, cudaMemcpyHostToDevice, s));
-    EF_CHECK(ef_launch_csr_dirichlet_rows(nRows, c->dCsrRows, c->dIndptr, c->dIndices, csrData, s));
-    EF_CUDA(cudaEventRecord(c->csrRowsDone, s));
-    return EF_OK;
+    const ef_status st = ef_launch_csr_dirichlet_rows(nRows, c->dCsrRows, c->dIndptr, c->dIndices, csrData, s);
+    EF_CUDA(cudaEventRecord(c->csrRowsDone, s));  // (the copy is under way in any case)
+    return st;
 }
 
 ef_status ef_set_dirichlet(ef_ctx* c, const int64_t* dofs, int64_t n) {

@@ -182,7 +182,8 @@ ef_status ef_csr_pattern(ef_ctx* ctx, int32_t* indptr, int32_t* indices);
  * stiffness (exported in FP64 first). */
 ef_status ef_update_csr(ef_ctx* ctx, const double* Kvij, double* csrData, void* stream);
 /* solvers/nonlinearimplicitstaticparallelmk2.pyx:66-109 applyDirichletK without the final
- * eliminate_zeros: rows (host [nRows]) zeroed, diagonal 1. */
+ * eliminate_zeros: rows (host [nRows], read before the call returns) zeroed, diagonal 1.  Stream ordered;
+ * EF_ERR_STATE under stream capture. */
 ef_status ef_csr_dirichlet_rows(ef_ctx* ctx, double* csrData, const int64_t* rows, int64_t nRows, void* stream);
 
 /* ---- fast path: 3x3-block (BSR) system assembled from the element blocks without
