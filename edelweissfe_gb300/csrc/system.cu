@@ -181,20 +181,34 @@ ef_status dot_host(ef_ctx* c, const double* a, const double* b, double* out, cud
     return EF_OK;
 }
 
-static ef_status pcg_plan(ef_ctx* c, int vDouble) {
-    if (c->pcgPlanned) return EF_OK;
-    PcgResidentPlan p;
-    ef_pcg_resident_plan(vDouble, c->nSM, (int)c->nNodes, c->hRowPtr0.data(), c->hColIdx0.data(), p);
-    if (p.smem > 0) {
-        EF_CHECK(upload(&c->dPcgHaloPtr, p.haloPtr));
-        EF_CHECK(upload(&c->dPcgHaloIdx, p.haloIdx));
-        EF_CHECK(upload(&c->dPcgGroupPtr, p.groupPtr));
-        EF_CHECK(upload(&c->dPcgLcol, p.lcol));
-    }
-    c->pcgSmem = p.smem;
-    c->pcgShape = p.shape;
+// A plan that finds no memory, on the host or the device, is none: the streaming kernel needs nothing beyond the
+// context's vectors (EF_PCG_RESIDENT=0 takes it always).
+static void pcg_plan(ef_ctx* c, int vDouble) {
+    if (c->pcgPlanned) return;
     c->pcgPlanned = true;
-    return EF_OK;
+    c->pcgSmem = 0;
+    const char* e = getenv("EF_PCG_RESIDENT");
+    if (e && atoi(e) == 0) return;
+    PcgResidentPlan p;
+    try {
+        ef_pcg_resident_plan(vDouble, c->nSM, (int)c->nNodes, c->hRowPtr0.data(), c->hColIdx0.data(), p);
+    } catch (const std::exception&) {
+        return;
+    }
+    if (p.smem == 0) return;
+    if (upload(&c->dPcgHaloPtr, p.haloPtr) == EF_OK && upload(&c->dPcgHaloIdx, p.haloIdx) == EF_OK &&
+        upload(&c->dPcgGroupPtr, p.groupPtr) == EF_OK && upload(&c->dPcgLcol, p.lcol) == EF_OK) {
+        c->pcgSmem = p.smem;
+        c->pcgShape = p.shape;
+        return;
+    }
+    (void)cudaGetLastError();
+    cudaFree(c->dPcgHaloPtr);
+    cudaFree(c->dPcgHaloIdx);
+    cudaFree(c->dPcgGroupPtr);
+    cudaFree(c->dPcgLcol);
+    c->dPcgHaloPtr = c->dPcgHaloIdx = c->dPcgGroupPtr = nullptr;
+    c->dPcgLcol = nullptr;
 }
 
 // one PCG launch on the free DOFs: solves K d = rhs (rhs zero on Dirichlet DOFs); vDouble: the
@@ -202,7 +216,7 @@ static ef_status pcg_plan(ef_ctx* c, int vDouble) {
 ef_status run_pcg(ef_ctx* c, int vDouble, const void* rhs, void* sol, int maxIter, double rtol,
                          PcgResult* out, ef_solve_info* prof, cudaStream_t s) {
     void** w = vDouble ? c->w64k : c->w32;
-    EF_CHECK(pcg_plan(c, vDouble));
+    pcg_plan(c, vDouble);
     pcg_result_clear(c->hRes->pcg);
     if (prof) EF_CUDA(cudaEventRecord(c->ev[0], s));
     if (c->pcgSmem > 0)
