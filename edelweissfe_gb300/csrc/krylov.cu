@@ -741,14 +741,16 @@ static void pcg_shape(int vDouble, int n, int nSM, PcgShape* p) {
     p->lpr = pcg_lanes((n + p->grid - 1) / p->grid, tpb, vDouble);
 }
 
-#define EF_PCG(K, T, ...) \
-    (lpr == 32 ? (const void*)K<T, 32, ##__VA_ARGS__> : (lpr == 16 ? (const void*)K<T, 16, ##__VA_ARGS__> : (lpr == 8 ? (const void*)K<T, 8, ##__VA_ARGS__> : (const void*)K<T, 4, ##__VA_ARGS__>)))
-static const void* pcg_kernel(int vDouble, int lpr) {
-    return vDouble ? EF_PCG(pcg_persistent_kernel, double) : EF_PCG(pcg_persistent_kernel, float);
-}
+// the lanes that pcg_lanes gives: 4 to 32 for FP32 vectors, 4 and 8 for FP64 ones
+#define EF_PCG(K, ...)                                                                                       \
+    (vDouble ? (lpr == 8 ? (const void*)K<double, 8, ##__VA_ARGS__> : (const void*)K<double, 4, ##__VA_ARGS__>) \
+     : lpr == 32 ? (const void*)K<float, 32, ##__VA_ARGS__>                                                  \
+     : lpr == 16 ? (const void*)K<float, 16, ##__VA_ARGS__>                                                  \
+     : lpr == 8  ? (const void*)K<float, 8, ##__VA_ARGS__>                                                   \
+                 : (const void*)K<float, 4, ##__VA_ARGS__>)
+static const void* pcg_kernel(int vDouble, int lpr) { return EF_PCG(pcg_persistent_kernel); }
 static const void* pcg_resident(int vDouble, int lpr, bool cluster) {
-    if (cluster) return vDouble ? EF_PCG(pcg_resident_kernel, double, true) : EF_PCG(pcg_resident_kernel, float, true);
-    return vDouble ? EF_PCG(pcg_resident_kernel, double, false) : EF_PCG(pcg_resident_kernel, float, false);
+    return cluster ? EF_PCG(pcg_resident_kernel, true) : EF_PCG(pcg_resident_kernel, false);
 }
 #undef EF_PCG
 
@@ -1019,6 +1021,11 @@ extern "C" ef_status ef_pcg_solve_noalloc(int64_t nNodes, const int32_t* rowPtr,
                 return EF_ERR_CUDA;
             }
             EF_CUDA(cudaDeviceGetAttribute(&g_noallocSMs[dev], cudaDevAttrMultiProcessorCount, dev));
+            // a kernel's code goes to the device when it is first used: all of them now, so that no later call does that
+            for (int lpr = 4; lpr <= 8; lpr *= 2) {
+                cudaFuncAttributes fa;
+                EF_CUDA(cudaFuncGetAttributes(&fa, pcg_kernel(1, lpr)));
+            }
             g_noallocPtr[dev] = p;
         }
     }
