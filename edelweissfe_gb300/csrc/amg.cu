@@ -1566,8 +1566,9 @@ int ef_amg_coarse_dofs() { return BC; }
 int ef_max_coarsest_nodes() { return kMaxCoarsestDof / BC; }
 
 // Warps per row of the 6-DOF levels' residual and post-smoothing: four for levels that a warp per row leaves with
-// less than about 13 warps an SM (preconditioner on the 300-node second level of 169,781 nodes 92.9 -> 91.6 us;
-// on the 6,664-node first level four warps cost 5.5 us)
+// less than about 13 warps an SM.  us of the preconditioner with one and with four, by nodes of the first coarse level: 233
+// 19.4 and 17.6, 1,260 33.5 and 31.8, 1,650 36.9 and 34.3, 2,110 41.6 and 40.7, 2,710 44.7 and 44.8, 3,740 51.3 and
+// 52.7, 4,740 59.9 and 60.9
 constexpr int kRowWarps = 4;
 static int row_warps(int nN) { return nN <= 2048 ? kRowWarps : 1; }
 

@@ -7,8 +7,9 @@ namespace ef {
 
 // Loads of matrix values and indices ahead of griddepcontrol.wait: a cycle's small kernels are chains of a few
 // dependent loads (row pointer, index, value, vector), and only the vector comes from the kernel before.  The
-// matrices are set-up results, and the kernel launched just before one of these is always one of the cycle or of the
-// Krylov iteration, so they are complete once the CTA can run.  Volatile, so that they stay ahead of the wait.  us of the
+// matrices are set-up results, and the kernel launched just before one of these never writes them (the rule at
+// launch_dep): it is one of the cycle or of the Krylov iteration, or in the power iteration the norm or the scaling of its
+// vector.  Volatile, so that they stay ahead of the wait.  us of the
 // cycle before and now: 7,412 nodes of quadratic elements 25.3 -> 23.2, hex8 4,225 nodes 19.3 -> 17.2, 11,849 nodes 27.7 ->
 // 23.5, 18,081 nodes 30.0 -> 25.5, 169,781 nodes 78.1 -> 71.3.
 __device__ __forceinline__ int early(const int32_t* p) {

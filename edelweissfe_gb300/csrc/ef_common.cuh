@@ -31,10 +31,15 @@ inline cudaStream_t counted(cudaStream_t s) {
 // Programmatic dependent launch of the kernels of the Krylov iteration and the multigrid cycle
 // (chains of short dependent kernels).  A kernel launched by launch_dep() may be scheduled while
 // the kernel before it in the stream is still running, so its launch latency and CTA
-// rasterisation overlap the predecessor's tail.  Such a kernel starts with dep_entry(): it waits
-// until the predecessor grid has completed and its writes are visible, before any load or
-// store, and then lets its own successor be scheduled.  Launched without the attribute (EF_PDL=0
+// rasterisation overlap the predecessor's tail.  Such a kernel calls dep_entry(): it waits
+// until the predecessor grid has completed and its writes are visible, before it stores anything or loads anything
+// that the predecessor writes, and then lets its own successor be scheduled.  Launched without the attribute (EF_PDL=0
 // or a predecessor that is not a kernel), both instructions return at once.
+// The rule for what a kernel may load ahead of dep_entry() (early.cuh, the small Gram-Schmidt kernels): nothing that the
+// kernel launched just before it on the stream writes.  What any earlier launch wrote is complete: the kernel before is
+// either an ordinary launch, which began after all of it, or itself past its wait before a successor is scheduled.  So a
+// kernel that rewrites matrix values, indices or basis vectors must not be the launch just before one of
+// these; with another launch between (set-up ends in block inverses and norms, a column in its axpy) it is safe.
 bool dep_launch_enabled();
 __device__ __forceinline__ void dep_entry() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");

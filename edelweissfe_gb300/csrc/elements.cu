@@ -14,9 +14,9 @@
 //
 // Thread mapping: TPE threads per element (8 for <= 8 Gauss points, 32
 // otherwise); thread `lane` of an element owns Gauss point `lane` for the
-// constitutive phase, node `lane` for the residual phase and node pairs
-// lane, lane+TPE, ... for the stiffness phase.  Per-element scratch lives in
-// shared memory; the state is structure-of-arrays [var][element*nQP + qp] so
+// constitutive phase and node `lane` for the residual phase; in the stiffness
+// phase the node pairs of all the CTA's elements are dealt out over its threads.
+// Per-element scratch lives in shared memory; the state is structure-of-arrays [var][element*nQP + qp] so
 // that the constitutive phase reads and writes it coalesced.
 
 #include <math.h>

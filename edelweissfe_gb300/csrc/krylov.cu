@@ -7,7 +7,8 @@
 // Dirichlet DOFs are eliminated symmetrically: every Krylov vector vanishes on them and
 // the operator's Dirichlet rows are masked to zero, so the free-free block is solved.
 // Reductions are deterministic (per-CTA partials summed in a fixed order by every CTA).
-// The persistent kernel is launched cooperatively (all CTAs resident); its waits are bounded.
+// The persistent kernels over a grid are launched cooperatively (all CTAs resident) and their waits are bounded; the form
+// that is one cluster is a plain launch that waits at the hardware's cluster barrier only.
 
 #include <algorithm>
 #include <cstdio>
@@ -117,9 +118,10 @@ __global__ void __launch_bounds__(kKB) bsr_residual_kernel(int nNodes, const int
 //  * one CTA per SM, and fewer when a CTA's lanes already cover the rows in one pass (pcg_shape).
 //  * the scalars of the recurrence belong to one thread of a CTA (grid_sum);
 //  * systems that fit into shared memory stay there (pcg_resident_kernel), small ones in one cluster.
-// us an iteration, before (304 CTAs, cooperative-groups barriers, rows dealt out over the grid, scalars in
-// every thread) and now: FP32, 624 nodes 20 -> 3.7, 4,836 nodes 23 -> 7.6, 23,000 nodes 26 -> 9.2; FP64,
-// 525 nodes 24 -> 7.8, 3,146 nodes 28 -> 12.
+// us an iteration (kernel time), before (304 CTAs, cooperative-groups barriers, rows dealt out over the grid, scalars in
+// every thread) and now: FP32, 624 nodes 21.4 -> 5.3, 4,836 nodes 23.7 -> 9.1, 22,491 nodes 28.3 -> 10.9; FP64,
+// 525 nodes 26.6 -> 7.9, 3,146 nodes 27.4 -> 11.8.  Streaming: FP32, 38,125 nodes 28.1 -> 19.7, 169,781 nodes 78.7 -> 63.3;
+// FP64, 22,491 nodes 48.4 -> 38.5, 169,781 nodes 222 -> 144.
 
 constexpr int kPcgMaxCtas = 160;                    // slots of a reduction (one CTA per SM)
 constexpr int kPcgMaxCluster = 16;                  // CTAs of the cluster form
@@ -141,8 +143,8 @@ struct PcgTpb {
 };
 
 // Sums beyond a warp and the scalars made of them are FP64 for FP32 vectors too (PcgScalars); an unevaluated pair
-// of FP32 numbers in their place saves 0.6 us of an iteration of 624 nodes, but carries 48 bits and
-// ends at FP32's range.
+// of FP32 numbers in their place saves 1.5 us of an iteration (624 nodes 5.3, 4,836 nodes 9.1), but carries 48 bits
+// and ends at FP32's range.
 // bits of a published sum: never kPcgEmpty
 __device__ __forceinline__ unsigned long long slot_bits(double v) {
     return v == v ? (unsigned long long)__double_as_longlong(v) : 0x7ff8000000000000ull;
@@ -729,9 +731,9 @@ ef_status ef_launch_bsr_residual(int nNodes, const int32_t* rowPtr, const int32_
 }
 
 // Lanes per block row, CTAs and slot sets of the PCG on n block rows.  Fewer CTAs make a reduction
-// cheaper and an iteration's work per SM larger: 128 rows a CTA in FP32 (4,836 nodes: 7.1 us an
-// iteration with 38 CTAs, 8.8 with 152) and 16 in FP64, whose pipe bounds the product (525 nodes: 9.8 us
-// with 33 CTAs, 11.6 with 132, 22 with 5), up to one CTA per SM.
+// cheaper and an iteration's work per SM larger: 128 rows a CTA in FP32 (4,836 nodes: 9.1 us an
+// iteration with 38 CTAs, 9.4 with 76, 10.1 with 152) and 16 in FP64, whose pipe bounds the product (525 nodes: 9.8 us
+// with 33 CTAs, 10.5 with 132, 22 with 5), up to one CTA per SM.
 static void pcg_shape(int vDouble, int n, int nSM, PcgShape* p) {
     const int tpb = vDouble ? PcgTpb<double>::value : PcgTpb<float>::value;
     const int least = vDouble ? 16 : 128;
@@ -830,8 +832,9 @@ static cudaLaunchConfig_t cluster_config(const PcgShape& shape, int vDouble, siz
 }
 
 // The rule of the dispatch.  A system that fits into one cluster's shared memory (about 3,200 rows of 27
-// blocks in FP32, 1,600 in FP64) runs there: a reduction through the cluster's barrier costs about a third
-// of one through L2.  Else one that fits into all SMs' shared memory runs in the grid form.  Else
+// blocks in FP32, 1,600 in FP64) runs there: a reduction through the cluster's barrier costs about half
+// of one through L2 (us an iteration in the cluster and in the grid form: FP32, 624 nodes 5.3 and 8.2, 2,730 nodes 6.2
+// and 8.6; FP64, 525 nodes 7.8 and 9.8, but 1,440 nodes, for which the FP64 pipes of 16 SMs are few, 12.9 and 10.6).  Else one that fits into all SMs' shared memory runs in the grid form.  Else
 // plan.smem is 0: the streaming kernel.
 void ef_pcg_resident_plan(int vDouble, int nSM, int nNodes, const int32_t* rowPtr, const int32_t* colIdx,
                           PcgResidentPlan& plan) {

@@ -79,7 +79,9 @@ static ef_status sell_build(ef_ctx* c) {
     // meet in shared memory).  us of the product / the preconditioner with 4, 8 and 16 warps: 4,225 nodes 8.5 / 23.4,
     // 8.4 / 21.2, 6.4 / 19.3; 18,081 nodes 8.6 / 35.7, 8.4 / 31.6, 8.4 / 29.9; 38,125 nodes 10.4 / 40.0, 9.0 / 36.9,
     // 10.5 / 38.0; 169,781 nodes 28.7 / 78.0, 26.8 / 79.9, 38.8 / 92.4; rows of quadratic elements (up to 81 blocks) at
-    // 7,412 nodes 20.7 / 38.0, 13.9 / 29.4, 10.5 / 25.3 (32 warps: the same)
+    // 7,412 nodes 20.7 / 38.0, 13.9 / 29.4, 10.5 / 25.3.  The product with 8, 16 and 32 warps, which long rows want where there
+    // are few slices: tied meshes of 328 nodes 8.3, 7.3, 6.5, of 6,754 nodes 12.4, 10.3, 8.7; quadratic elements of 605
+    // nodes 8.4, 8.2, 8.0; hex8 4,225 nodes 8.2, 6.3, 6.4
     const int perSM = (n0 + 32 * c->nSM - 1) / (32 * c->nSM);  // slices
     const int warps = perSM <= 6 ? 16 : (perSM <= 24 ? 8 : 4);
     c->sellSplit = split(getenv("EF_SELL_SPLIT"), warps);

@@ -254,10 +254,11 @@ __global__ void __launch_bounds__(sell_split_threads(S)) sell_spmv3_kernel(
 }
 
 // The product in the diagonal form from half the matrix.  K is symmetric to the bit (both blocks of a pair of
-// nodes sum the same element blocks in the same order), so only the diagonals j >= diaN / 2 are stored: the block of
+// nodes sum the same element blocks in the same order; where ties or collapsed elements give a pair several blocks of one
+// element, to the rounding of that sum), so only the diagonals j >= diaN / 2 are stored: the block of
 // diagonal -d in row r is the transpose of the one of diagonal d in row r - d, which the rows a little
 // further up have just brought into L1 and L2.  The order of a row's sums is the full form's: the same bits.
-// Half the values leave HBM 86 MB of them at 169,781 nodes (full form 165 MB) and L2 the rest.  STREAM (above 60,000 nodes, where
+// Half the values leave HBM (86 MB of them at 169,781 nodes, full form 165 MB) and L2 the rest.  STREAM (above 60,000 nodes, where
 // an iteration's matrices no longer fit into L2 and would evict the basis): the blocks are marked for early eviction
 // and taken two at a time; below, one after the other from cached lines (11,849 nodes: 6.7 us against 7.5 two at a
 // time, 38,125 nodes: 9.1 against 10.4).  us of a product, full form and now: 11,849 nodes 8.3 -> 6.7, 38,125 nodes

@@ -179,7 +179,7 @@ ef_status ef_export_vij(ef_ctx* ctx, double* Kvij, void* stream);
 ef_status ef_csr_pattern(ef_ctx* ctx, int32_t* indptr, int32_t* indices);
 /* data[s] = sum of Kvij[k] over the VIJ pairs k of slot s, added in increasing k from 0.0:
  * bit-identical to the reference's serial loop.  Kvij = NULL uses the context's own element
- * stiffness (exported in FP64 first). */
+ * stiffness, taken from its blocks with the same result as from the vector that ef_export_vij writes. */
 ef_status ef_update_csr(ef_ctx* ctx, const double* Kvij, double* csrData, void* stream);
 /* solvers/nonlinearimplicitstaticparallelmk2.pyx:66-109 applyDirichletK without the final
  * eliminate_zeros: rows (host [nRows], read before the call returns) zeroed, diagonal 1.  Stream ordered;
