@@ -80,3 +80,29 @@ def test_solves_without_the_sliced_copy(gpu_lib, monkeypatch, sizes):
             assert torch.cuda.mem_get_info()[0] >= free
             assert torch.equal(x, _solve(s, b))
         _lib.check(s.lib.ef_batch_setup(s.ctx, s.nProb, s.nodePtr.ctypes.data), "ef_batch_setup")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [0, 1, 2, 3, 4, 5, 6])
+def test_problems_without_nodes(gpu_lib, tile):
+    """Empty node ranges among the others, and enough of them that clusters take only such problems."""
+    from edelweissfe_gb300 import _lib
+
+    s, b = _batch([2, 5, 1])
+    _lib.check(s.lib.ef_batch_set_tile(s.ctx, tile), "ef_batch_set_tile")
+    x = _solve(s, b)
+    ptr = np.concatenate([[0], s.nodePtr, np.full(400, s.nodePtr[-1])]).astype(np.int32)  # 401 empty ones
+    n = len(ptr) - 1
+    its = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    rel = torch.full((n,), -1.0, dtype=torch.float64, device="cuda")
+    out = torch.full((n, 3), -1.0, dtype=torch.float64, device="cuda")
+    y = s._vec()
+    _lib.check(s.lib.ef_batch_setup(s.ctx, n, ptr.ctypes.data), "ef_batch_setup")
+    _lib.check(s.lib.ef_batch_solve(s.ctx, 1e-10, 20000, b.data_ptr(), y.data_ptr(), its.data_ptr(), rel.data_ptr(),
+                                    s._stream()), "ef_batch_solve")  # fmt: skip
+    _lib.check(s.lib.ef_batch_norms(s.ctx, b.data_ptr(), b.data_ptr(), None, out.data_ptr(), s._stream()), "ef_batch_norms")
+    its, rel, out = its.cpu().numpy(), rel.cpu().numpy(), out.cpu().numpy()
+    some = np.diff(ptr) > 0
+    assert (its[some] > 0).all() and (rel[some] <= 1e-10).all() and (out[some, 0] > 0).all()
+    assert not its[~some].any() and not rel[~some].any() and not out[~some].any()
+    assert float((x - y).norm() / x.norm()) <= 1e-6  # (another cluster size may sum in another order)
